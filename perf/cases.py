@@ -153,20 +153,21 @@ def _groups(t, ldims):
     return list(out.values())      # in order of first appearance
 
 
-def _decaying_state(meta, g):
+def _decaying_state(meta, seed):
     """A two-site state whose singular values fall off exponentially in every block-matrix (no two
     alike), between random orthonormal vectors."""
-    buf = torch.zeros(max(meta.size, 1), dtype=torch.float64, device="cuda")
+    rng = np.random.default_rng(seed)
+    data = np.zeros(meta.size)
     for i, x in enumerate(_groups(meta, 2)):
         k = min(x["m"], x["n"])
-        at = torch.arange(k, dtype=torch.float64, device="cuda") + (0.618034 * i) % 1.0
-        left = torch.linalg.qr(torch.randn(x["m"], k, dtype=torch.float64, device="cuda", generator=g))[0]
-        right = torch.linalg.qr(torch.randn(x["n"], k, dtype=torch.float64, device="cuda", generator=g))[0]
-        dense = (left * torch.exp(at * (-7.0 / k))) @ right.T
+        at = np.arange(k) + (0.618034 * i) % 1.0
+        left = np.linalg.qr(rng.standard_normal((x["m"], k)))[0]
+        right = np.linalg.qr(rng.standard_normal((x["n"], k)))[0]
+        dense = (left * np.exp(at * (-7.0 / k))) @ right.T
         for b, r, c, m, n in x["blk"]:
             o = int(meta.offsets[b])
-            buf[o:o + m * n] = dense[r:r + m, c:c + n].reshape(-1)
-    return DTensor(_meta(meta), buf)
+            data[o:o + m * n] = dense[r:r + m, c:c + n].reshape(-1)
+    return DTensor.from_host(BSTensor(meta.legs, meta.coords, meta.dtype, data))
 
 
 ENV_AXES = [[[0], [0]], [[0, 2], [0, 1]], [[0, 3, 1], [0, 1, 2]]]
@@ -198,7 +199,7 @@ def _inputs(case, seed):
     if kind in ("matvec", "lanczos"):
         return [DTensor.from_host(t) for t in _chain(case["D"], int(seed) % 1000003)]
     if kind == "svd":
-        return [_decaying_state(_chain_psi(case["D"]), g)]
+        return [_decaying_state(_chain_psi(case["D"]), int(seed))]
     if kind == "qr":
         return [_normal(_qr_layout(case["blocks"], case["lo"], case["hi"]), g)]
     m = _chain_psi(case["D"])

@@ -157,7 +157,7 @@ QLTG_API int qltg_ctrct_plan_destroy(qltg_ctrct_plan* plan);
 
 /* Schedule of a plan's grouped GEMM stage. No counterpart in the reference, which issues one
  * cublasDgemm per task (framework/hp_numeric/blas_level3.h:797-856) and has no schedule.
- * f64_tile_rows: rows of the FP64 output tiles, 32 or 64 (x 32 columns); 0 keeps it.
+ * f64_tile_rows: rows of the FP64 output tiles of four warps, 32 or 64 (x 16 columns); 0 keeps it.
  * split_stack: split-precision row stacking (output blocks with the same task structure share
  * 128-row tiles), 1 on, 0 off, -1 keeps it. Rebuilds the affected schedule (allocates and
  * synchronises `stream`; not inside a stream capture). Results are the same under every

@@ -268,7 +268,7 @@ int qltg_ctrct_plan_set_schedule(qltg_ctrct_plan* plan, int32_t f64_tile_rows, i
     QLTG_CUDA(cudaSetDevice(plan->p.ctx->device));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     CtrctPlan& p = plan->p;
-    if (f64_tile_rows) set_f64_tile(p, f64_tile_rows, 32, s);
+    if (f64_tile_rows) set_f64_tile(p, f64_tile_rows, s);
     if (split_stack >= 0) {
       TuneChoice c;
       c.f64_bm = p.sched.bm;

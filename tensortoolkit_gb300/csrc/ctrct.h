@@ -65,6 +65,13 @@ struct GemmTile {
   int32_t cblk;
   int16_t tm, tn;
 };
+// FP64 warp tiles of one output block with the same extent inside the block (the block's
+// interior, its right edge, its bottom edge, the corner): tile t of the launch, begin <= t, is
+// tile (tm0 + l / tn_count, tn0 + l % tn_count) with l = t - begin.
+struct GemmTileRun {
+  int32_t cblk, begin;
+  int32_t tm0, tn0, tn_count;
+};
 struct GemmRowChunk {          // skinny output blocks: 256 consecutive rows of one block
   int32_t cblk;
   int32_t chunk;
@@ -82,10 +89,12 @@ struct SkinnyFuse {
 struct GemmSchedule {
   std::vector<GemmCBlk> cblk;
   std::vector<GemmTask> task;
-  std::vector<GemmTile> tile;           // 64 x 64 tiles (DMMA / DFMA kernels)
+  std::vector<GemmTileRun> run;         // FP64 warp tiles, longest first
+  int64_t ntiles = 0;                   // tiles of all runs
+  bool share_tiles = false;             // a CTA's warps share each tile (few or very long tiles)
   std::vector<GemmRowChunk> skinny;     // row chunks of skinny blocks (n, k <= 8)
-  DevBuf d_cblk, d_task, d_tile, d_skinny, d_counter;
-  int bm = 32, bn = 32;
+  DevBuf d_cblk, d_task, d_run, d_skinny, d_counter;
+  int bm = 32;                          // rows of the FP64 tiles of a CTA's four warps
   int skinny_maxn = 8;                  // largest n of the skinny blocks (kernel variant)
 };
 
@@ -212,13 +221,14 @@ void plan_contraction(CtrctPlan& p, cudaStream_t s);
 TuneChoice tune_plan(CtrctPlan& p, const void* a, const void* b, void* c, int mode, cudaStream_t s, bool* cached);
 void apply_choice(CtrctPlan& p, int mode, const TuneChoice& c, cudaStream_t s);
 uint64_t plan_signature(const CtrctPlan& p, int mode);
-void set_f64_tile(CtrctPlan& p, int bm, int bn, cudaStream_t s);
+void set_f64_tile(CtrctPlan& p, int bm, cudaStream_t s);
 // Grouped-GEMM schedule, operand transposes and device buffers of a planned contraction.
 void finalize_plan(CtrctPlan& p, cudaStream_t s);
 int64_t exec_launches_split(const CtrctPlan& p);
 void exec_contraction(CtrctPlan& p, const void* a, const void* b, void* c, int mode, cudaStream_t s, int stage = 0);
 
 // grouped GEMM launchers (gemm_f64.cu)
+constexpr int kF64TileCols = 16;   // columns of an FP64 warp tile
 bool skinny_cblk(const GemmSchedule& g, int32_t q);
 int skinny_rows_per_item();
 // Grid of the skinny kernel: one full wave of resident CTAs (the first call queries the

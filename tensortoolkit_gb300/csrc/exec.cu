@@ -7,37 +7,59 @@
 
 namespace qltg {
 
-// FP64 output tiles of g.bm x g.bn, longest first (the DFMA kernel takes them in this order).
-static void f64_tile_list(GemmSchedule& g) {
-  g.tile.clear();
-  struct Cand { GemmTile t; int64_t cost; };
+// FP64 warp tiles (bm / 4 rows x kF64TileCols columns, gemm_f64.cu), longest first. All tiles of
+// a block with the same extent inside it cost the same, so the list holds at most four runs per
+// block instead of every tile.
+static void f64_tile_list(GemmSchedule& g, int num_sms) {
+  g.run.clear();
+  g.ntiles = 0;
+  struct Cand { GemmTileRun r; int64_t count, cost; };
   std::vector<Cand> cands;
+  const int rows = g.bm / 4, cols = kF64TileCols;
+  // multiply-adds issued for an extent: whole 8 x 4 pieces
+  auto padded = [](int64_t r, int64_t c) { return ((r + 7) / 8 * 8) * ((c + 3) / 4 * 4); };
   for (int32_t q = 0; q < (int32_t)g.cblk.size(); ++q) {
     const GemmCBlk& cb = g.cblk[q];
     if (skinny_cblk(g, q)) continue;
+    QLTG_CHECK((cb.m + 31) / 32 < 32768 && (cb.n + 31) / 32 < 32768, QLTG_ERR_UNSUPPORTED,
+               "output block too large for the tile grid");
     int64_t ksum = 0;
     for (int32_t t = cb.t0; t < cb.t1; ++t) ksum += g.task[t].k;
-    const int tm = (cb.m + g.bm - 1) / g.bm, tn = (cb.n + g.bn - 1) / g.bn;
-    QLTG_CHECK(tm < 32768 && tn < 32768, QLTG_ERR_UNSUPPORTED, "output block too large for the tile grid");
-    for (int i = 0; i < tm; ++i)
-      for (int j = 0; j < tn; ++j) {
-        const int64_t rows = std::min(g.bm, cb.m - i * g.bm), cols = std::min(g.bn, cb.n - j * g.bn);
-        cands.push_back({GemmTile{q, (int16_t)i, (int16_t)j}, ksum * rows * cols});
-      }
+    const int fm = cb.m / rows, fn = cb.n / cols, em = cb.m % rows, en = cb.n % cols;
+    auto add = [&](int tm0, int tn0, int nm, int nn, int r, int c) {
+      if (nm > 0 && nn > 0) cands.push_back({GemmTileRun{q, 0, tm0, tn0, nn}, (int64_t)nm * nn, ksum * padded(r, c)});
+    };
+    add(0, 0, fm, fn, rows, cols);
+    add(0, fn, fm, en ? 1 : 0, rows, en);
+    add(fm, 0, em ? 1 : 0, fn, em, cols);
+    add(fm, fn, em ? 1 : 0, en ? 1 : 0, em, en);
   }
   std::stable_sort(cands.begin(), cands.end(), [](const Cand& x, const Cand& y) { return x.cost > y.cost; });
-  g.tile.reserve(cands.size());
-  for (auto& c : cands) g.tile.push_back(c.t);
+  // Tiles are shared by a CTA's four warps when the longest one, alone on its sub-partition,
+  // would take more than a quarter of a sub-partition's share of the launch (four per SM): with
+  // four warps resident on each, one such tile then ends the launch late. All or none: sharing
+  // only the longest ones left the rest to start late (FP64 step 3 of the matvec: D = 1000 280 us
+  // own / 266 us shared / 362-449 us mixed, D = 300 82 / 51 us; steps above the line, D = 4000:
+  // 2.52-2.58 ms own, 2.75-2.78 ms shared).
+  double total = 0;
+  for (auto& c : cands) total += (double)c.cost * c.count;
+  g.share_tiles = !cands.empty() && 4.0 * cands[0].cost > total / (4.0 * std::max(1, num_sms));
+  g.run.reserve(cands.size());
+  for (auto& c : cands) {
+    QLTG_CHECK(g.ntiles + c.count < ((int64_t)1 << 31) - (1 << 20), QLTG_ERR_UNSUPPORTED, "too many output tiles");
+    c.r.begin = (int32_t)g.ntiles;
+    g.ntiles += c.count;
+    g.run.push_back(c.r);
+  }
 }
 
-void set_f64_tile(CtrctPlan& p, int bm, int bn, cudaStream_t s) {
-  QLTG_CHECK((bm == 32 && bn == 32) || (bm == 64 && bn == 32), QLTG_ERR_INVALID, "FP64 tiles are 32 x 32 or 64 x 32");
+void set_f64_tile(CtrctPlan& p, int bm, cudaStream_t s) {
+  QLTG_CHECK(bm == 32 || bm == 64, QLTG_ERR_INVALID, "FP64 tiles have 32 or 64 rows");
   GemmSchedule& g = p.sched;
-  if (g.bm == bm && g.bn == bn && g.d_tile.get()) return;
+  if (g.bm == bm && g.d_run.get()) return;
   g.bm = bm;
-  g.bn = bn;
-  f64_tile_list(g);
-  g.d_tile = upload(g.tile, s);
+  f64_tile_list(g, p.ctx->num_sms);
+  g.d_run = upload(g.run, s);
   QLTG_CUDA(cudaStreamSynchronize(s));
 }
 
@@ -53,14 +75,14 @@ void finalize_plan(CtrctPlan& p, cudaStream_t s) {
       for (int32_t c = 0; c * (int64_t)rows_per_item < cb.m; ++c) g.skinny.push_back(GemmRowChunk{q, c});
     }
   }
-  f64_tile_list(g);
+  f64_tile_list(g, p.ctx->num_sms);
   // Operand transposes. A task reads its operand block from the transposed scratch unless
   // (a) the permutation leaves the block's layout unchanged, or (b) it is a skinny task and
   // the block, read in place, is a strided matrix (rows and columns each one stride); such
   // tasks read the operand itself (offset flag kFromSrc) and blocks nobody reads from the
   // scratch get no transpose work.
   const size_t eb = p.a.elem_bytes();
-  const bool any_work = !g.tile.empty() || !g.skinny.empty();
+  const bool any_work = g.ntiles || !g.skinny.empty();
   std::vector<uint8_t> skinny_task(g.task.size(), 0);
   for (int32_t q = 0; q < (int32_t)g.cblk.size(); ++q)
     if (skinny_cblk(g, q))
@@ -134,10 +156,10 @@ void finalize_plan(CtrctPlan& p, cudaStream_t s) {
   if (!g.skinny.empty()) (void)skinny_grid((int)g.skinny.size(), p.a.dtype == QLTG_C128, g.skinny_maxn, p.ctx->num_sms);
   g.d_cblk = upload(g.cblk, s);
   g.d_task = upload(g.task, s);
-  g.d_tile = upload(g.tile, s);
+  g.d_run = upload(g.run, s);
   g.d_skinny = upload(g.skinny, s);
   g.d_counter.alloc(sizeof(int));
-  p.launches_per_exec = (g.tile.empty() ? 0 : 2) + (g.skinny.empty() ? 0 : 1) +   // memset + GEMM
+  p.launches_per_exec = (g.ntiles ? 2 : 0) + (g.skinny.empty() ? 0 : 1) +   // memset + GEMM
                          (p.a_tl.ntiles ? 1 : 0) + (p.b_tl.ntiles ? 1 : 0);
   QLTG_CUDA(cudaStreamSynchronize(s));
 }
@@ -151,7 +173,7 @@ int64_t exec_launches_split(const CtrctPlan& p) {
 }
 
 void exec_contraction(CtrctPlan& p, const void* a, const void* b, void* c, int mode, cudaStream_t s, int stage) {
-  if (p.sched.tile.empty() && p.sched.skinny.empty()) return;
+  if (!p.sched.ntiles && p.sched.skinny.empty()) return;
   QLTG_CHECK(a && b && c, QLTG_ERR_INVALID, "null device buffer");
   QLTG_CHECK(stage >= 0 && stage <= 3, QLTG_ERR_INVALID, "stage must be 0, 1, 2 or 3");
   QLTG_CHECK(mode == QLTG_MODE_FP64 || mode == QLTG_MODE_SPLIT, QLTG_ERR_INVALID, "unknown arithmetic mode");

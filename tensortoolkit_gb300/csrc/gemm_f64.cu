@@ -3,16 +3,15 @@
 // Replaces the reference's serial loop of one cblas_dgemm / cublasDgemm per task with
 // beta = 0 for the first task of an output block and beta = 1 after it
 // (global_operations.h:895-992 -> raw_data_operations.h:530-548 -> blas_level3.h:35-56,
-// :797-856). Every output tile is owned by one CTA that loops over all tasks of its output
+// :797-856). Every output tile is owned by one warp that loops over all tasks of its output
 // block, accumulating sign_t * A_t[tile rows, :] B_t[:, tile cols] in registers, and stores
 // the tile once: no read-modify-write of C, no atomics, deterministic.
 //
 // Two kernels, chosen per output block when the plan is built:
-//  * k_gemm_dfma   - FP64 / complex128 (4 real FMAs per complex FMA) on 32 x 32 output tiles.
-//                    On this GPU the FP64 tensor path (mma.sync m8n8k4 f64) runs at the same
-//                    rate as DFMA (about 1.05 TFLOP/s each, measured) but pads every block to
-//                    8 x 8 x 4 fragments (48 % useful on the matvec's block shapes), so the
-//                    predicated DFMA tile is the faster FP64 kernel;
+//  * k_gemm_f64    - FP64 / complex128 (4 real FMAs per complex FMA) on warp tiles. On this
+//                    GPU the FP64 tensor path (mma.sync m8n8k4 f64) runs at the same rate as
+//                    DFMA (about 1.05 TFLOP/s each, measured) but pads every block to 8 x 8 x 4
+//                    fragments, so predicated DFMA is the faster FP64 kernel;
 //  * k_gemm_skinny - output blocks with n <= 8 and k <= 8 (the MPO steps of the two-site
 //                    matvec: m up to 3e4, k, n <= 3): one thread per output row, operand B
 //                    in registers, memory-streaming.
@@ -23,7 +22,9 @@
 namespace qltg {
 namespace {
 
-constexpr int NT = 256;
+constexpr int NT = 128;            // threads of an FP64 GEMM CTA: one warp per sub-partition
+// 16 warps per SM hide the operand latency (2 / 3 / 4 CTAs at D = 4000: 3.02 / 2.60 / 2.52 ms)
+constexpr int kF64CtasPerSm = 4;
 
 __device__ __forceinline__ void fma_acc(double& acc, double a, double b) { acc = fma(a, b, acc); }
 __device__ __forceinline__ void fma_acc(double2& acc, double2 a, double2 b) {
@@ -41,177 +42,131 @@ __device__ __forceinline__ double flip(double x, unsigned long long m) {
 __device__ __forceinline__ double2 flip(double2 x, unsigned long long m) { return make_double2(flip(x.x, m), flip(x.y, m)); }
 __device__ __forceinline__ unsigned long long sign_mask(int sign) { return sign < 0 ? 0x8000000000000000ull : 0ull; }
 
-constexpr int BM = 32, BN = 32, BK = 32;
-
-// 32 x 32 output tiles (BM = BN = 32): one output tile per work item; 16 x 16 threads, each 2 x 2 outputs at
-// (ty + 16 i, tx + 16 j). Operand tiles are staged through shared memory (A transposed so
-// a warp reads one broadcast row); outputs outside the block are predicated off so no FP64
-// issue slot is spent on padding. Work items are taken longest-first from an atomic
-// counter (the plan zeroes it before each launch), so the few very long tiles start first
-// and the rest fill in behind them.
-template <typename T>
-__global__ void __launch_bounds__(NT) k_gemm_dfma32(const GemmCBlk* __restrict__ cblk, const GemmTask* __restrict__ task,
-                                                  const GemmTile* __restrict__ tiles, int ntiles,
-                                                  const T* __restrict__ A, const T* __restrict__ As,
-                                                  const T* __restrict__ B, const T* __restrict__ Bs,
-                                                  T* __restrict__ C, int* __restrict__ counter) {
-  __shared__ T sA[BK][BM + 1];
-  __shared__ T sB[BK][BN];
-  __shared__ int s_ti;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  while (true) {
-    if (threadIdx.x == 0) s_ti = atomicAdd(counter, 1);
-    __syncthreads();
-    const int ti = s_ti;
-    __syncthreads();
-    if (ti >= ntiles) break;
-    const GemmTile tl = tiles[ti];
-    const GemmCBlk cb = cblk[tl.cblk];
-    const int r0 = tl.tm * BM, c0 = tl.tn * BN;
-    const int m = cb.m, n = cb.n;
-    T acc[2][2];
+// One task added to a warp's 8 TM x 4 TN tile: lane (lr, lc) of the warp's 8 x 4 grid holds the
+// outputs (lr + 8 i, lc + 4 j). Operands go straight from L1 / L2 into registers, U values of k
+// ahead of their use (the next values of an A row share its cache line; four B columns are one
+// sector).
+template <typename T, int TM, int TN>
+__device__ __forceinline__ void f64_tile_task(T (&acc)[TM][TN], const T* __restrict__ a, const T* __restrict__ b, int k,
+                                              int n, unsigned long long sg, const int (&row)[TM],
+                                              const int (&col)[TN], const bool (&rv)[TM], const bool (&cv)[TN]) {
+  constexpr int U = (sizeof(T) == 8 ? 4 : 2) * (TN == 1 ? 2 : 1);
+  T av[U][TM], bv[U][TN];
+  auto load = [&](int k0) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int u = 0; u < U; ++u) {
+      const int kk = min(k0 + u, k - 1);
 #pragma unroll
-      for (int j = 0; j < 2; ++j) acc[i][j] = zero_of(T());
-    bool rv[2], cv[2];
+      for (int i = 0; i < TM; ++i) av[u][i] = __ldg(a + (int64_t)row[i] * k + kk);
 #pragma unroll
-    for (int i = 0; i < 2; ++i) { rv[i] = r0 + ty + 16 * i < m; cv[i] = c0 + tx + 16 * i < n; }
-    for (int t = cb.t0; t < cb.t1; ++t) {
-      const GemmTask tk = task[t];
-      const int k = tk.k;
-      const T* a = operand_block(A, As, tk.a_off);
-      const T* b = operand_block(B, Bs, tk.b_off);
-      const unsigned long long sg = sign_mask(tk.sign);
-      for (int k0 = 0; k0 < k; k0 += BK) {
-        const int kc = min(BK, k - k0);
-#pragma unroll
-        for (int e = threadIdx.x; e < BM * BK; e += NT) {
-          const int row = e / BK, kk = e % BK;
-          T v = zero_of(T());
-          if (kk < kc && r0 + row < m) v = flip(a[(int64_t)(r0 + row) * k + k0 + kk], sg);
-          sA[kk][row] = v;
-        }
-#pragma unroll
-        for (int e = threadIdx.x; e < BK * BN; e += NT) {
-          const int kk = e / BN, col = e % BN;
-          T v = zero_of(T());
-          if (kk < kc && c0 + col < n) v = b[(int64_t)(k0 + kk) * n + c0 + col];
-          sB[kk][col] = v;
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int kk = 0; kk < kc; ++kk) {
-          const T a0 = sA[kk][ty], a1 = sA[kk][ty + 16];
-          const T b0 = sB[kk][tx], b1 = sB[kk][tx + 16];
-          if (rv[0]) {
-            if (cv[0]) fma_acc(acc[0][0], a0, b0);
-            if (cv[1]) fma_acc(acc[0][1], a0, b1);
-          }
-          if (rv[1]) {
-            if (cv[0]) fma_acc(acc[1][0], a1, b0);
-            if (cv[1]) fma_acc(acc[1][1], a1, b1);
-          }
-        }
-        __syncthreads();
-      }
+      for (int j = 0; j < TN; ++j) bv[u][j] = __ldg(b + (int64_t)kk * n + col[j]);
     }
+  };
+  load(0);
+  for (int k0 = 0; k0 < k; k0 += U) {
+    T ac[U][TM], bc[U][TN];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int u = 0; u < U; ++u) {
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
-        if (rv[i] && cv[j]) C[cb.c_off + (int64_t)(r0 + ty + 16 * i) * n + c0 + tx + 16 * j] = acc[i][j];
+      for (int i = 0; i < TM; ++i) ac[u][i] = flip(av[u][i], sg);
+#pragma unroll
+      for (int j = 0; j < TN; ++j) bc[u][j] = bv[u][j];
+    }
+    if (k0 + U < k) load(k0 + U);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k0 + u < k) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j)
+            if (rv[i] && cv[j]) fma_acc(acc[i][j], ac[u][i], bc[u][j]);
+      }
   }
 }
 
-// k depth of one shared-memory stage: 32, or 16 where the two operand tiles would pass the
-// 48 KB of static shared memory (complex 64-row tiles).
-template <typename T, int BM, int BN>
-constexpr int dfma_bk() { return (int)sizeof(T) * 32 * (BM + 1 + BN) <= 48 * 1024 ? 32 : 16; }
-
-// One output tile of BM x BN per work item (BM = 16 TM, BN = 16 TN); 16 x 16 threads, each
-// TM x TN outputs at (ty + 16 i, tx + 16 j). Operand tiles are staged through shared memory
-// (A transposed so a warp reads one broadcast row); outputs outside the block are predicated
-// off so no FP64 issue slot is spent on padding. Work items are taken longest-first from an
-// atomic counter (the plan zeroes it before each launch), so the few very long tiles start
-// first and the rest fill in behind them. Used for 64 x 32 tiles (TM = 4, TN = 2): the
-// taller tile reads each staged operand value for twice the FMAs; the 32 x 32 tile above
-// pads less on small blocks. The tuner picks between them per plan.
+// All tasks of an output block added up for the tile of 8 TM rows and 4 TN columns at (r0, c0),
+// by one warp, and stored.
 template <typename T, int TM, int TN>
-__global__ void __launch_bounds__(NT, TM * TN <= 4 ? 4 : 2) k_gemm_dfma(const GemmCBlk* __restrict__ cblk, const GemmTask* __restrict__ task,
-                                                  const GemmTile* __restrict__ tiles, int ntiles,
-                                                  const T* __restrict__ A, const T* __restrict__ As,
-                                                  const T* __restrict__ B, const T* __restrict__ Bs,
-                                                  T* __restrict__ C, int* __restrict__ counter) {
-  constexpr int BM = 16 * TM, BN = 16 * TN, BK = dfma_bk<T, BM, BN>();
-  __shared__ T sA[BK][BM + 1];
-  __shared__ T sB[BK][BN];
-  __shared__ int s_ti;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  while (true) {
-    if (threadIdx.x == 0) s_ti = atomicAdd(counter, 1);
-    __syncthreads();
-    const int ti = s_ti;
-    __syncthreads();
-    if (ti >= ntiles) break;
-    const GemmTile tl = tiles[ti];
-    const GemmCBlk cb = cblk[tl.cblk];
-    const int r0 = tl.tm * BM, c0 = tl.tn * BN;
-    const int m = cb.m, n = cb.n;
-    T acc[TM][TN];
+__device__ __forceinline__ void f64_tile(const GemmCBlk& cb, const GemmTask* __restrict__ task, int r0, int c0, int lane,
+                                         const T* __restrict__ A, const T* __restrict__ As, const T* __restrict__ B,
+                                         const T* __restrict__ Bs, T* __restrict__ C) {
+  const int lr = lane >> 2, lc = lane & 3, m = cb.m, n = cb.n;
+  bool rv[TM], cv[TN];   // pieces inside the block (warp-uniform)
+  int row[TM], col[TN];  // this lane's rows and columns, clamped into the block
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+  for (int i = 0; i < TM; ++i) {
+    rv[i] = r0 + 8 * i < m;
+    row[i] = min(r0 + 8 * i + lr, m - 1);
+  }
 #pragma unroll
-      for (int j = 0; j < TN; ++j) acc[i][j] = zero_of(T());
-    bool rv[TM], cv[TN];
+  for (int j = 0; j < TN; ++j) {
+    cv[j] = c0 + 4 * j < n;
+    col[j] = min(c0 + 4 * j + lc, n - 1);
+  }
+  T acc[TM][TN];
 #pragma unroll
-    for (int i = 0; i < TM; ++i) rv[i] = r0 + ty + 16 * i < m;
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) cv[j] = c0 + tx + 16 * j < n;
-    for (int t = cb.t0; t < cb.t1; ++t) {
-      const GemmTask tk = task[t];
-      const int k = tk.k;
-      const T* a = operand_block(A, As, tk.a_off);
-      const T* b = operand_block(B, Bs, tk.b_off);
-      const unsigned long long sg = sign_mask(tk.sign);
-      for (int k0 = 0; k0 < k; k0 += BK) {
-        const int kc = min(BK, k - k0);
+    for (int j = 0; j < TN; ++j) acc[i][j] = zero_of(T());
+  for (int t = cb.t0; t < cb.t1; ++t) {
+    const GemmTask tk = task[t];
+    f64_tile_task<T, TM, TN>(acc, operand_block(A, As, tk.a_off), operand_block(B, Bs, tk.b_off), tk.k, n,
+                             sign_mask(tk.sign), row, col, rv, cv);
+  }
 #pragma unroll
-        for (int e = threadIdx.x; e < BM * BK; e += NT) {
-          const int row = e / BK, kk = e % BK;
-          T v = zero_of(T());
-          if (kk < kc && r0 + row < m) v = flip(a[(int64_t)(r0 + row) * k + k0 + kk], sg);
-          sA[kk][row] = v;
-        }
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int e = threadIdx.x; e < BK * BN; e += NT) {
-          const int kk = e / BN, col = e % BN;
-          T v = zero_of(T());
-          if (kk < kc && c0 + col < n) v = b[(int64_t)(k0 + kk) * n + c0 + col];
-          sB[kk][col] = v;
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int kk = 0; kk < kc; ++kk) {
-          T av[TM], bv[TN];
-#pragma unroll
-          for (int i = 0; i < TM; ++i) av[i] = sA[kk][ty + 16 * i];
-#pragma unroll
-          for (int j = 0; j < TN; ++j) bv[j] = sB[kk][tx + 16 * j];
-#pragma unroll
-          for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN; ++j)
-              if (rv[i] && cv[j]) fma_acc(acc[i][j], av[i], bv[j]);
-        }
-        __syncthreads();
-      }
+    for (int j = 0; j < TN; ++j) {
+      const int r = r0 + 8 * i + lr, c = c0 + 4 * j + lc;
+      if (r < m && c < n) C[cb.c_off + (int64_t)r * n + c] = acc[i][j];
     }
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j)
-        if (rv[i] && cv[j]) C[cb.c_off + (int64_t)(r0 + ty + 16 * i) * n + c0 + tx + 16 * j] = acc[i][j];
+}
+
+// Output tiles of 8 TM x 16. The FP64 pipe takes about 20 SM cycles per warp instruction and
+// each of the four sub-partitions has its own quarter of it, so what decides this kernel is how
+// evenly the multiply-adds spread over the sub-partitions and how few of them are padding;
+// operand reads are cheap beside that. Hence a warp owns a tile (no CTA-wide barrier), pieces of
+// 8 x 4 outputs outside the block are skipped by a warp-uniform test (at most 7 rows and 3
+// columns of padding), and tiles are taken longest-first from an atomic counter (zeroed before
+// the launch). One warp alone needs 320 cycles per k; where that makes the longest tile too long
+// for the launch (share_tiles), a CTA's four warps share each tile, four columns each.
+// Measured (D = 4000 matvec steps 0 and 3): 2.52 and 2.58 ms = 1.03 and 1.01 of cuBLAS DGEMM's
+// 1.1 TFLOP/s, against 2.91 and 3.19 ms for 32 x 32 tiles of a CTA staged in shared memory;
+// D = 1000: 258 and 266 us against 318 and 392 us (launch, transposes and skinny blocks included).
+template <typename T, int TM, bool SHARE>
+__global__ void __launch_bounds__(NT) k_gemm_f64(const GemmCBlk* __restrict__ cblk, const GemmTask* __restrict__ task,
+                                                 const GemmTileRun* __restrict__ runs, int nruns, int ntiles,
+                                                 const T* __restrict__ A, const T* __restrict__ As,
+                                                 const T* __restrict__ B, const T* __restrict__ Bs,
+                                                 T* __restrict__ C, int* __restrict__ counter) {
+  constexpr int TN = kF64TileCols / 4;
+  static_assert(NT / 32 == TN, "a shared tile has one piece column per warp");
+  __shared__ int s_ti;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  while (true) {
+    int ti = 0;
+    if (SHARE) {
+      __syncthreads();   // everyone has read s_ti
+      if (threadIdx.x == 0) s_ti = atomicAdd(counter, 1);
+      __syncthreads();
+      ti = s_ti;
+    } else {
+      if (lane == 0) ti = atomicAdd(counter, 1);
+      ti = __shfl_sync(0xffffffffu, ti, 0);
+    }
+    if (ti >= ntiles) break;
+    int lo = 0, hi = nruns - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (__ldg(&runs[mid].begin) <= ti) lo = mid; else hi = mid - 1;
+    }
+    const GemmTileRun run = runs[lo];
+    const GemmCBlk cb = cblk[run.cblk];
+    const int l = ti - run.begin, lm = l / run.tn_count;
+    const int r0 = (run.tm0 + lm) * (8 * TM), c0 = (run.tn0 + l - lm * run.tn_count) * kF64TileCols;
+    if constexpr (!SHARE) f64_tile<T, TM, TN>(cb, task, r0, c0, lane, A, As, B, Bs, C);
+    else if (c0 + 4 * warp < cb.n) f64_tile<T, TM, 1>(cb, task, r0, c0 + 4 * warp, lane, A, As, B, Bs, C);
   }
 }
 
@@ -403,23 +358,24 @@ void launch_skinny_t(const GemmSchedule& g, const Operands& op, void* c, int gri
                                                    static_cast<T*>(c), fuse, fields);
 }
 
-template <typename T, int TM, int TN>
-void launch_dfma_tile(const GemmSchedule& g, const Operands& op, void* c, int grid, cudaStream_t s) {
-  k_gemm_dfma<T, TM, TN><<<grid, NT, 0, s>>>(g.d_cblk.as<GemmCBlk>(), g.d_task.as<GemmTask>(), g.d_tile.as<GemmTile>(),
-                                             (int)g.tile.size(), static_cast<const T*>(op.a),
-                                             static_cast<const T*>(op.a_src), static_cast<const T*>(op.b),
-                                             static_cast<const T*>(op.b_src), static_cast<T*>(c), g.d_counter.as<int>());
+template <typename T, int TM, bool SHARE>
+void launch_f64_t(const GemmSchedule& g, const Operands& op, void* c, int num_sms, cudaStream_t s) {
+  const int64_t per_cta = SHARE ? 1 : NT / 32;
+  const int grid = (int)std::min<int64_t>((g.ntiles + per_cta - 1) / per_cta, (int64_t)std::max(1, num_sms) * kF64CtasPerSm);
+  k_gemm_f64<T, TM, SHARE><<<grid, NT, 0, s>>>(
+      g.d_cblk.as<GemmCBlk>(), g.d_task.as<GemmTask>(), g.d_run.as<GemmTileRun>(), (int)g.run.size(), (int)g.ntiles,
+      static_cast<const T*>(op.a), static_cast<const T*>(op.a_src), static_cast<const T*>(op.b),
+      static_cast<const T*>(op.b_src), static_cast<T*>(c), g.d_counter.as<int>());
 }
 
 template <typename T>
-void launch_dfma_t(const GemmSchedule& g, const Operands& op, void* c, int grid, cudaStream_t s) {
+void launch_f64(const GemmSchedule& g, const Operands& op, void* c, int num_sms, cudaStream_t s) {
   if (g.bm == 64) {
-    launch_dfma_tile<T, 4, 2>(g, op, c, grid, s);
+    if (g.share_tiles) launch_f64_t<T, 2, true>(g, op, c, num_sms, s);
+    else launch_f64_t<T, 2, false>(g, op, c, num_sms, s);
   } else {
-    k_gemm_dfma32<T><<<grid, NT, 0, s>>>(g.d_cblk.as<GemmCBlk>(), g.d_task.as<GemmTask>(), g.d_tile.as<GemmTile>(),
-                                         (int)g.tile.size(), static_cast<const T*>(op.a),
-                                         static_cast<const T*>(op.a_src), static_cast<const T*>(op.b),
-                                         static_cast<const T*>(op.b_src), static_cast<T*>(c), g.d_counter.as<int>());
+    if (g.share_tiles) launch_f64_t<T, 1, true>(g, op, c, num_sms, s);
+    else launch_f64_t<T, 1, false>(g, op, c, num_sms, s);
   }
 }
 
@@ -464,17 +420,12 @@ void launch_gemm_f64_skinny(const GemmSchedule& g, const Operands& op, void* c, 
 }
 
 void launch_gemm_f64(const GemmSchedule& g, const Operands& op, void* c, bool cplx, int num_sms, cudaStream_t s) {
-  const int nt = (int)g.tile.size();
   launch_gemm_f64_skinny(g, op, c, cplx, num_sms, s);
-  if (nt) {
-    QLTG_CUDA(cudaMemsetAsync(g.d_counter.get(), 0, sizeof(int), s));
-    const int grid = std::min(nt, std::max(1, num_sms) * 4);
-    if (cplx)
-      launch_dfma_t<double2>(g, op, c, grid, s);
-    else
-      launch_dfma_t<double>(g, op, c, grid, s);
-    QLTG_CUDA(cudaGetLastError());
-  }
+  if (!g.ntiles) return;
+  QLTG_CUDA(cudaMemsetAsync(g.d_counter.get(), 0, sizeof(int), s));
+  if (cplx) launch_f64<double2>(g, op, c, num_sms, s);
+  else launch_f64<double>(g, op, c, num_sms, s);
+  QLTG_CUDA(cudaGetLastError());
 }
 
 // ------------------------------------------------------------------ FP64 rate self-test

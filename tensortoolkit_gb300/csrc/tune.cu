@@ -3,8 +3,8 @@
 // The reference issues one cublasDgemm per task (framework/hp_numeric/blas_level3.h:797-856)
 // and has no schedule to choose. Here all tasks of a contraction go out in one persistent
 // launch, and how they are cut into tiles is a choice that depends on the block shapes:
-//  * FP64 (DFMA) tiles of 32 x 32 or 64 x 32 outputs - the taller tile reuses each staged
-//    operand value for twice the FMAs, the smaller one wastes less on small blocks;
+//  * FP64 warp tiles of 8 or 16 rows (32 or 64 per CTA) x 16 columns - the taller tile reads
+//    each operand value for twice the FMAs, the smaller one spreads the work more evenly;
 //  * split precision: row stacking on or off - stacking packs the A blocks of output blocks
 //    with the same task structure into shared 128-row tiles (less padding, one row-map load
 //    per output row), off keeps one block per tile.
@@ -85,7 +85,7 @@ uint64_t plan_signature(const CtrctPlan& p, int mode) {
 
 void apply_choice(CtrctPlan& p, int mode, const TuneChoice& c, cudaStream_t s) {
   if (mode == QLTG_MODE_FP64) {
-    set_f64_tile(p, c.f64_bm, 32, s);
+    set_f64_tile(p, c.f64_bm, s);
   } else {
     QLTG_CHECK(!(p.split && (p.split->a_static || p.split->b_static)), QLTG_ERR_INVALID,
                "the split schedule of a plan with operands packed once cannot change");

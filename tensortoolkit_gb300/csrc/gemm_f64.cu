@@ -45,25 +45,27 @@ __device__ __forceinline__ unsigned long long sign_mask(int sign) { return sign 
 // One task added to a warp's 8 TM x 4 TN tile: lane (lr, lc) of the warp's 8 x 4 grid holds the
 // outputs (lr + 8 i, lc + 4 j). Operands go straight from L1 / L2 into registers, U values of k
 // ahead of their use (the next values of an A row share its cache line; four B columns are one
-// sector).
+// sector). A predicated-off FP64 instruction takes as long as an executed one (78 cycles on its
+// sub-partition, measured), so nothing here is predicated: tiles are instantiated per number of
+// pieces inside the block, and a task's last k % U values run in a loop of their own.
 template <typename T, int TM, int TN>
 __device__ __forceinline__ void f64_tile_task(T (&acc)[TM][TN], const T* __restrict__ a, const T* __restrict__ b, int k,
                                               int n, unsigned long long sg, const int (&row)[TM],
-                                              const int (&col)[TN], const bool (&rv)[TM], const bool (&cv)[TN]) {
-  constexpr int U = (sizeof(T) == 8 ? 4 : 2) * (TN == 1 ? 2 : 1);
+                                              const int (&col)[TN]) {
+  constexpr int U = (sizeof(T) == 8 ? 4 : 2) * (TN == 1 ? 2 : 1) / TM;
   T av[U][TM], bv[U][TN];
   auto load = [&](int k0) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int kk = min(k0 + u, k - 1);
 #pragma unroll
-      for (int i = 0; i < TM; ++i) av[u][i] = __ldg(a + (int64_t)row[i] * k + kk);
+      for (int i = 0; i < TM; ++i) av[u][i] = __ldg(a + (int64_t)row[i] * k + k0 + u);
 #pragma unroll
-      for (int j = 0; j < TN; ++j) bv[u][j] = __ldg(b + (int64_t)kk * n + col[j]);
+      for (int j = 0; j < TN; ++j) bv[u][j] = __ldg(b + (int64_t)(k0 + u) * n + col[j]);
     }
   };
-  load(0);
-  for (int k0 = 0; k0 < k; k0 += U) {
+  int k0 = 0;
+  if (U <= k) load(0);
+  for (; k0 + U <= k; k0 += U) {
     T ac[U][TM], bc[U][TN];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -72,38 +74,41 @@ __device__ __forceinline__ void f64_tile_task(T (&acc)[TM][TN], const T* __restr
 #pragma unroll
       for (int j = 0; j < TN; ++j) bc[u][j] = bv[u][j];
     }
-    if (k0 + U < k) load(k0 + U);
+    if (k0 + 2 * U <= k) load(k0 + U);
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (k0 + u < k) {
 #pragma unroll
-        for (int i = 0; i < TM; ++i)
+      for (int i = 0; i < TM; ++i)
 #pragma unroll
-          for (int j = 0; j < TN; ++j)
-            if (rv[i] && cv[j]) fma_acc(acc[i][j], ac[u][i], bc[u][j]);
-      }
+        for (int j = 0; j < TN; ++j) fma_acc(acc[i][j], ac[u][i], bc[u][j]);
+  }
+#pragma unroll 1
+  for (; k0 < k; ++k0) {
+    T ac[TM], bc[TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i) ac[i] = flip(__ldg(a + (int64_t)row[i] * k + k0), sg);
+#pragma unroll
+    for (int j = 0; j < TN; ++j) bc[j] = __ldg(b + (int64_t)k0 * n + col[j]);
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) fma_acc(acc[i][j], ac[i], bc[j]);
   }
 }
 
 // All tasks of an output block added up for the tile of 8 TM rows and 4 TN columns at (r0, c0),
-// by one warp, and stored.
+// every 8 x 4 piece of which holds outputs of the block, by one warp, and stored. A function of
+// its own: inlined side by side the sizes' prefetch registers spill.
 template <typename T, int TM, int TN>
-__device__ __forceinline__ void f64_tile(const GemmCBlk& cb, const GemmTask* __restrict__ task, int r0, int c0, int lane,
+__device__ __noinline__ void f64_tile(const GemmCBlk& cb, const GemmTask* __restrict__ task, int r0, int c0, int lane,
                                          const T* __restrict__ A, const T* __restrict__ As, const T* __restrict__ B,
                                          const T* __restrict__ Bs, T* __restrict__ C) {
   const int lr = lane >> 2, lc = lane & 3, m = cb.m, n = cb.n;
-  bool rv[TM], cv[TN];   // pieces inside the block (warp-uniform)
   int row[TM], col[TN];  // this lane's rows and columns, clamped into the block
 #pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    rv[i] = r0 + 8 * i < m;
-    row[i] = min(r0 + 8 * i + lr, m - 1);
-  }
+  for (int i = 0; i < TM; ++i) row[i] = min(r0 + 8 * i + lr, m - 1);
 #pragma unroll
-  for (int j = 0; j < TN; ++j) {
-    cv[j] = c0 + 4 * j < n;
-    col[j] = min(c0 + 4 * j + lc, n - 1);
-  }
+  for (int j = 0; j < TN; ++j) col[j] = min(c0 + 4 * j + lc, n - 1);
   T acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
@@ -112,7 +117,7 @@ __device__ __forceinline__ void f64_tile(const GemmCBlk& cb, const GemmTask* __r
   for (int t = cb.t0; t < cb.t1; ++t) {
     const GemmTask tk = task[t];
     f64_tile_task<T, TM, TN>(acc, operand_block(A, As, tk.a_off), operand_block(B, Bs, tk.b_off), tk.k, n,
-                             sign_mask(tk.sign), row, col, rv, cv);
+                             sign_mask(tk.sign), row, col);
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i)
@@ -123,25 +128,37 @@ __device__ __forceinline__ void f64_tile(const GemmCBlk& cb, const GemmTask* __r
     }
 }
 
+// The tile at (r0, c0), as wide as the block leaves it (up to kF64TileCols columns).
+template <typename T, int TM>
+__device__ __forceinline__ void f64_tile_cols(const GemmCBlk& cb, const GemmTask* __restrict__ task, int r0, int c0,
+                                              int lane, const T* __restrict__ A, const T* __restrict__ As,
+                                              const T* __restrict__ B, const T* __restrict__ Bs, T* __restrict__ C) {
+  const int n = cb.n - c0;
+  if (n > 12) f64_tile<T, TM, 4>(cb, task, r0, c0, lane, A, As, B, Bs, C);
+  else if (n > 8) f64_tile<T, TM, 3>(cb, task, r0, c0, lane, A, As, B, Bs, C);
+  else if (n > 4) f64_tile<T, TM, 2>(cb, task, r0, c0, lane, A, As, B, Bs, C);
+  else f64_tile<T, TM, 1>(cb, task, r0, c0, lane, A, As, B, Bs, C);
+}
+
 // Output tiles of 8 TM x 16. The FP64 pipe takes about 20 SM cycles per warp instruction and
 // each of the four sub-partitions has its own quarter of it, so what decides this kernel is how
 // evenly the multiply-adds spread over the sub-partitions and how few of them are padding;
-// operand reads are cheap beside that. Hence a warp owns a tile (no CTA-wide barrier), pieces of
-// 8 x 4 outputs outside the block are skipped by a warp-uniform test (at most 7 rows and 3
+// operand reads are cheap beside that. Hence a warp owns a tile (no CTA-wide barrier), a tile at a
+// block's edge is run at the size of the 8 x 4 pieces that hold outputs (at most 7 rows and 3
 // columns of padding), and tiles are taken longest-first from an atomic counter (zeroed before
 // the launch). One warp alone needs 320 cycles per k; where that makes the longest tile too long
 // for the launch (share_tiles), a CTA's four warps share each tile, four columns each.
-// Measured (D = 4000 matvec steps 0 and 3): 2.52 and 2.58 ms = 1.03 and 1.01 of cuBLAS DGEMM's
-// 1.1 TFLOP/s, against 2.91 and 3.19 ms for 32 x 32 tiles of a CTA staged in shared memory;
-// D = 1000: 258 and 266 us against 318 and 392 us (launch, transposes and skinny blocks included).
+// Measured (D = 4000 matvec steps 0 and 3): 2.44 and 2.45 ms = 1.07 of cuBLAS DGEMM's 1.1
+// TFLOP/s, against 2.91 and 3.19 ms for 32 x 32 tiles of a CTA staged in shared memory, and 2.52
+// and 2.58 ms with the pieces outside a block predicated off; D = 1000: 231 and 252 us against
+// 318 and 392 us (launch, transposes and skinny blocks included).
 template <typename T, int TM, bool SHARE>
-__global__ void __launch_bounds__(NT) k_gemm_f64(const GemmCBlk* __restrict__ cblk, const GemmTask* __restrict__ task,
+__global__ void __launch_bounds__(NT, sizeof(T) == 8 ? (TM == 1 ? 4 : 3) : 2) k_gemm_f64(const GemmCBlk* __restrict__ cblk, const GemmTask* __restrict__ task,
                                                  const GemmTileRun* __restrict__ runs, int nruns, int ntiles,
                                                  const T* __restrict__ A, const T* __restrict__ As,
                                                  const T* __restrict__ B, const T* __restrict__ Bs,
                                                  T* __restrict__ C, int* __restrict__ counter) {
-  constexpr int TN = kF64TileCols / 4;
-  static_assert(NT / 32 == TN, "a shared tile has one piece column per warp");
+  static_assert(NT / 32 == kF64TileCols / 4, "a shared tile has one piece column per warp");
   __shared__ int s_ti;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   while (true) {
@@ -165,8 +182,15 @@ __global__ void __launch_bounds__(NT) k_gemm_f64(const GemmCBlk* __restrict__ cb
     const GemmCBlk cb = cblk[run.cblk];
     const int l = ti - run.begin, lm = l / run.tn_count;
     const int r0 = (run.tm0 + lm) * (8 * TM), c0 = (run.tn0 + l - lm * run.tn_count) * kF64TileCols;
-    if constexpr (!SHARE) f64_tile<T, TM, TN>(cb, task, r0, c0, lane, A, As, B, Bs, C);
-    else if (c0 + 4 * warp < cb.n) f64_tile<T, TM, 1>(cb, task, r0, c0 + 4 * warp, lane, A, As, B, Bs, C);
+    if constexpr (SHARE) {
+      if (c0 + 4 * warp >= cb.n) continue;
+      if (TM > 1 && r0 + 8 >= cb.m) f64_tile<T, 1, 1>(cb, task, r0, c0 + 4 * warp, lane, A, As, B, Bs, C);
+      else f64_tile<T, TM, 1>(cb, task, r0, c0 + 4 * warp, lane, A, As, B, Bs, C);
+    } else if (TM > 1 && r0 + 8 >= cb.m) {
+      f64_tile_cols<T, 1>(cb, task, r0, c0, lane, A, As, B, Bs, C);
+    } else {
+      f64_tile_cols<T, TM>(cb, task, r0, c0, lane, A, As, B, Bs, C);
+    }
   }
 }
 

@@ -8,26 +8,31 @@
 
 namespace qltg {
 
-// One block permutation for the batched transpose kernel (dst-order dims after
-// squeezing unit dims and merging runs that stay adjacent).
+// One block permutation for the batched transpose kernel (transpose.cu), cut into work items of
+// one warp each. Dims are those left after squeezing unit dims and merging runs that stay
+// adjacent; offsets inside a block are below 2^31.
+enum PermMode : int32_t { kPermWhole = 0, kPermTile = 1, kPermRuns = 2 };
 struct PermDesc {
   int64_t src_off, dst_off;
-  int64_t sstride[kMaxRank];   // source stride of each destination dim
-  int32_t dims[kMaxRank];      // destination-order dims
-  int32_t rank;
-  int32_t p;                   // destination dim that is innermost in the source (-1: gather mode)
-  int32_t tp, tq;              // tile extents along p and along the innermost dst dim
-  int32_t tiles_p, tiles_q;    // tiles along p and along the innermost dst dim
-  int32_t u, tu, tiles_u;      // batched outer dim (-1: none), its tile extent and tile count
-  int64_t nouter;              // product of the remaining dims (gather mode: block size)
   int64_t tile_begin;          // first global work item of this block
   uint64_t sign_mask;          // 0, or the sign bit: the block's +-1 sign applied by XOR
+  int32_t mode;
+  int32_t nd;                  // entries of dims / sstr / dstr
+  // whole: every dim (dstr: their reciprocals), runs: the dims outside a run, both in destination
+  // order; tile: the dims outside a tile
+  uint32_t dims[kMaxRank], sstr[kMaxRank], dstr[kMaxRank];
+  // tile: up to two source-inner dims p0 (stride 1 in the source), p1 and two destination-inner
+  // dims q0 (stride 1 in the destination), q1: extents, extents of a tile, tiles
+  uint32_t np[2], ep[2], tp[2], dp[2];   // dp: destination strides of p0, p1
+  uint32_t nq[2], eq[2], tq[2], sq[2];   // sq: source strides of q0, q1
+  uint32_t size;               // whole: elements; runs: elements of a run
+  uint32_t per;                // runs: runs per item (1: an item is a piece of a run)
 };
 
 struct TransposeList {
   std::vector<PermDesc> host;
   std::vector<uint8_t> identity;   // per block: its data layout is unchanged by the permutation
-  DevBuf dev;
+  DevBuf dev;                      // descriptors, then the block of every work item
   int64_t ntiles = 0;
   int64_t nblocks = 0;
   // skip_identity: blocks whose layout the permutation leaves unchanged get no work (the

@@ -5,400 +5,344 @@
 // framework/hp_numeric/ten_trans.h:56-114, :245-349) and the ±1 block sign of
 // BlockSparseDataTensor::Transpose (global_operations.h:393-441).
 //
-// Per block, unit dims are squeezed and destination-adjacent dims that are also adjacent
-// in the source are merged. If the innermost destination dim is also innermost in the
-// source, the block is a set of contiguous runs copied with 16-byte vector accesses;
-// otherwise tiles over (source-innermost dim p, destination-innermost dim q) are staged
-// through shared memory so both the read (along p) and the write (along q) are coalesced.
-// Tiles are 32 x 32, or Tp x Tq (x Tu of one batched outer dim) up to 32 KB of data when one
-// of the two dims is short (an inner dim of 4 elements gets 4 x 256 tiles, whose reads and
-// writes are still long contiguous runs). A CTA reads its next tile into a second shared
-// buffer (cp.async, no staging registers) while it writes the current one out, so a tile's
-// worth of loads is always in flight. Only blocks whose two inner dims are both short fall
-// back to a destination-ordered gather. The +-1 block sign is applied by flipping the sign
-// bit (no floating-point multiply). Each CTA takes a contiguous range of work items, so it
-// looks up its first block once and then walks forward.
+// Per block, unit dims are squeezed and destination-adjacent dims that are also adjacent in the
+// source are merged. What is left is cut into work items of one warp each (8 KB of data), which
+// need no CTA-wide barrier and have all their loads in flight at once, 20 warps per SM:
+//  * tile: a box over the source-inner dims P (one, or two when the first is short) and the
+//    destination-inner dims Q (likewise), about 32 x 32, read along P and written along Q through
+//    shared memory (rows an odd number of elements apart: no bank conflicts). Two dims on a side
+//    keep the runs long when the innermost extent is 3 (an MPO bond): P and Q index ranges are
+//    contiguous in the source and in the destination;
+//  * whole: a block of up to 8 KB that no single tile covers, read and written as one flat range;
+//  * runs: the innermost dim is the same on both sides, so runs (or pieces of long ones) are
+//    copied, a flat range of as many runs as make 8 KB.
+// The +-1 block sign is applied by flipping the sign bit (no floating-point multiply). Bound by
+// HBM: lenv . psi at D = 4000 (80 MB) reversed 32.9 us = 0.71 of the measured copy rate, 107 us
+// with CTA-wide tiles of power-of-two extents; the 5544 blocks of a complex Hubbard psi (20 MB,
+// from L2) 8.2 us, 57 us before - there the descriptor and data latencies of one item bound it.
 #include <algorithm>
-#include <mutex>
 #include <string>
+#include <tuple>
 
 #include "ctrct.h"
 
 namespace qltg {
 namespace {
 
-constexpr int kTile = 32;
-constexpr int kTileMax = 4096;    // elements per batched tile (Tp * Tq * Tu), 8-byte elements
-constexpr int kRunChunk = 4096;   // elements per copy-mode / gather-mode work item
-constexpr int kPermThreads = 256;
-constexpr int kLoadBatch = 8;     // copy-mode loads issued per thread before storing
-
-// Tile budget in elements: the same 32 KB of data per tile for real and complex elements.
-__host__ __device__ constexpr int tile_budget(int elem_bytes) { return elem_bytes == 16 ? kTileMax / 2 : kTileMax; }
-// One tile buffer in elements: Tu planes of Tq rows of Tp + 1 (Tp >= 2): at most 1.5x the tile.
-__host__ __device__ constexpr int tile_buf_elems(int elem_bytes) { return tile_budget(elem_bytes) * 3 / 2; }
-
-template <typename T>
-__device__ __forceinline__ void cp_async_elem(T* dst, const T* src) {
-  if constexpr (sizeof(T) == 8)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
-  else
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+constexpr int kPermWarps = 4;      // per CTA
+constexpr int kPermThreads = 32 * kPermWarps;
+constexpr int kPermCtasPerSm = 5;   // 3 / 4 / 5 / 6 / 8 (smaller tiles): 34.8 / 32.9 / 32.9 / 38.7 / 41.2 us at D = 4000 (below)
+// Elements of one warp's buffer: 32 rows of 33 FP64 values, or as many bytes of complex ones.
+// Small enough that division by an extent is a multiplication (see inv_of).
+__host__ __device__ constexpr int perm_cap(int elem_bytes) { return elem_bytes == 16 ? 528 : 1056; }
 
 __device__ __forceinline__ double flip(double x, uint64_t m) {
   return __longlong_as_double(__double_as_longlong(x) ^ (long long)m);
 }
 __device__ __forceinline__ double2 flip(double2 x, uint64_t m) { return make_double2(flip(x.x, m), flip(x.y, m)); }
 
-// A tile-mode work item, decoded: a Tp x Tq x Tu tile over (p, q, u) (u: one outer dim batched
-// so a tile holds up to the budget even when the inner dims are short).
-template <typename T>
-struct TileJob {
-  const T* s;
-  T* o;
-  uint32_t sq, su, dp, du;
-  int np, nq, ulim, ip0, iq0;
-  int tp, tq, tu, lp, lq, lu, n;
-  bool u_next;
-  uint64_t sg;
-};
+// e / d for e, d <= 1056 (the largest buffer) as (e inv_of(d)) >> 21: the product is below 2^32, and
+// rounding the reciprocal up adds less than e / 2^21 to the quotient, which is below 1 / d.
+__host__ __device__ __forceinline__ uint32_t inv_of(uint32_t d) { return ((1u << 21) + d - 1) / d; }
+__device__ __forceinline__ uint32_t div_by(uint32_t e, uint32_t inv) { return (e * inv) >> 21; }
 
-__host__ __device__ inline bool is_tile_item(const PermDesc& d) { return d.rank > 0 && d.p >= 0 && d.p != d.rank - 1; }
-
-template <typename T>
-__device__ __forceinline__ TileJob<T> tile_job(const PermDesc& d, int64_t local, const T* src, T* dst) {
-  TileJob<T> j;
-  const int r = d.rank, q = r - 1;
-  j.tp = d.tp;
-  j.tq = d.tq;
-  j.tu = d.tu;
-  const uint32_t per_outer = (uint32_t)d.tiles_p * (uint32_t)d.tiles_q * (uint32_t)d.tiles_u;
-  const uint32_t outer = (uint32_t)local / per_outer;
-  uint32_t tt = (uint32_t)local - outer * per_outer;
-  const uint32_t tui = tt / ((uint32_t)d.tiles_p * (uint32_t)d.tiles_q);
-  tt -= tui * ((uint32_t)d.tiles_p * (uint32_t)d.tiles_q);
-  const uint32_t tpi = tt / (uint32_t)d.tiles_q;
-  j.ip0 = (int)(tpi * (uint32_t)j.tp);
-  j.iq0 = (int)((tt - tpi * (uint32_t)d.tiles_q) * (uint32_t)j.tq);
-  const int u0 = (int)(tui * (uint32_t)j.tu);
-  uint32_t rem = outer, soff = 0, doff = 0, dstr = 1, dp = 0, du = 0;
-  for (int i = r - 1; i >= 0; --i) {
-    const uint32_t di = (uint32_t)d.dims[i];
-    if (i == d.p) dp = dstr;
-    if (i == d.u) du = dstr;
-    if (i != d.p && i != q && i != d.u) {
-      const uint32_t qq = rem / di;
-      const uint32_t x = rem - qq * di;
-      rem = qq;
-      soff += x * (uint32_t)d.sstride[i];
-      doff += x * dstr;
-    }
-    dstr *= di;
-  }
-  const int nu = d.u >= 0 ? d.dims[d.u] : 1;
-  j.su = d.u >= 0 ? (uint32_t)d.sstride[d.u] : 0u;
-  j.dp = dp;
-  j.du = du;
-  j.s = src + d.src_off + soff + (uint32_t)u0 * j.su;
-  j.o = dst + d.dst_off + doff + (uint32_t)u0 * du;
-  j.np = d.dims[d.p];
-  j.nq = d.dims[q];
-  j.sq = (uint32_t)d.sstride[q];
-  j.lp = __ffs(j.tp) - 1;   // tile extents are powers of two
-  j.lq = __ffs(j.tq) - 1;
-  j.lu = __ffs(j.tu) - 1;
-  j.n = j.tp * j.tq * j.tu;
-  j.ulim = nu - u0;
-  // write order: q fastest (stride 1 in the destination), then whichever of u and p has the
-  // smaller destination stride (a short q dim with u next to it in the destination)
-  j.u_next = d.u >= 0 && du < dp;
-  j.sg = d.sign_mask;
-  return j;
-}
-
-// read into a tile buffer: p fastest (stride 1 in the source), straight into shared memory
-// (cp.async), so a whole tile is in flight per CTA without staging registers. With Tp <= the
-// CTA size a thread keeps one column pi and walks the (q, u) rows of the tile, so the index
-// arithmetic per element is a few integer operations.
-template <typename T>
-__device__ __forceinline__ void tile_loads(const TileJob<T>& j, T* buf) {
-  const int row = j.tp + 1, plane = j.tq * row;
-  if (j.tp <= kPermThreads) {
-    const int pi = threadIdx.x & (j.tp - 1);
-    if (j.ip0 + pi >= j.np) return;
-    const T* sb = j.s + (uint32_t)(j.ip0 + pi);
-    const int rstep = kPermThreads >> j.lp, nrows = j.tq * j.tu;
-    for (int ri = threadIdx.x >> j.lp; ri < nrows; ri += rstep) {
-      const int qi = ri & (j.tq - 1), ui = ri >> j.lq;
-      if (j.iq0 + qi < j.nq && ui < j.ulim)
-        cp_async_elem(buf + (ui * plane + qi * row + pi), sb + ((uint32_t)(j.iq0 + qi) * j.sq + (uint32_t)ui * j.su));
-    }
-    return;
-  }
-  for (int e = threadIdx.x; e < j.n; e += kPermThreads) {
-    const int pi = e & (j.tp - 1), qi = (e >> j.lp) & (j.tq - 1), ui = e >> (j.lp + j.lq);
-    if (j.ip0 + pi < j.np && j.iq0 + qi < j.nq && ui < j.ulim)
-      cp_async_elem(buf + (ui * plane + qi * row + pi),
-                    j.s + ((uint32_t)(j.ip0 + pi) + (uint32_t)(j.iq0 + qi) * j.sq + (uint32_t)ui * j.su));
-  }
-}
-
-// write out of a tile buffer in the write order (q fastest, then u or p); with Tq <= the CTA
-// size a thread keeps one q and walks the (p, u) columns
-template <typename T>
-__device__ __forceinline__ void tile_stores(const TileJob<T>& j, const T* buf) {
-  const int row = j.tp + 1, plane = j.tq * row;
-  if (j.tq <= kPermThreads) {
-    const int qi = threadIdx.x & (j.tq - 1);
-    if (j.iq0 + qi >= j.nq) return;
-    T* ob = j.o + (uint32_t)(j.iq0 + qi);
-    const int cstep = kPermThreads >> j.lq, ncols = j.tp * j.tu;
-    for (int ci = threadIdx.x >> j.lq; ci < ncols; ci += cstep) {
-      const int pi = j.u_next ? ci >> j.lu : ci & (j.tp - 1);
-      const int ui = j.u_next ? ci & (j.tu - 1) : ci >> j.lp;
-      if (j.ip0 + pi < j.np && ui < j.ulim)
-        ob[(uint32_t)(j.ip0 + pi) * j.dp + (uint32_t)ui * j.du] = flip(buf[ui * plane + qi * row + pi], j.sg);
-    }
-    return;
-  }
-  for (int e = threadIdx.x; e < j.n; e += kPermThreads) {
-    const int qi = e & (j.tq - 1);
-    const int pi = j.u_next ? (e >> (j.lq + j.lu)) & (j.tp - 1) : (e >> j.lq) & (j.tp - 1);
-    const int ui = j.u_next ? (e >> j.lq) & (j.tu - 1) : e >> (j.lp + j.lq);
-    if (j.ip0 + pi < j.np && j.iq0 + qi < j.nq && ui < j.ulim)
-      j.o[(uint32_t)(j.iq0 + qi) + (uint32_t)(j.ip0 + pi) * j.dp + (uint32_t)ui * j.du] =
-          flip(buf[ui * plane + qi * row + pi], j.sg);
+// Source and destination offsets of index `rem` over the descriptor's dims (last fastest).
+__device__ __forceinline__ void outer_offsets(const PermDesc& d, uint32_t rem, uint32_t& soff, uint32_t& doff) {
+  soff = doff = 0;
+  for (int i = d.nd - 1; i >= 0; --i) {
+    const uint32_t di = d.dims[i], q = rem / di, x = rem - q * di;
+    rem = q;
+    soff += x * d.sstr[i];
+    doff += x * d.dstr[i];
   }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kPermThreads) k_permute(const PermDesc* __restrict__ descs, int nd, int64_t ntiles,
+__device__ __forceinline__ void cp_async_elem(T* dst, const T* src) {
+  if constexpr (sizeof(T) == 8)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <typename T>
+__global__ void __launch_bounds__(kPermThreads, kPermCtasPerSm) k_permute(const PermDesc* __restrict__ descs, int nd,
+                                                          const int32_t* __restrict__ item_block, int64_t nitems,
                                                           const T* __restrict__ src, T* __restrict__ dst) {
-  // two tile buffers: Tu planes of Tq rows of Tp + 1 (Tp a power of two, so the row stride
-  // is odd); tile t + 1 is read into one while tile t is written out of the other
-  extern __shared__ __align__(16) uint8_t perm_smem[];
-  T* const bufs = reinterpret_cast<T*>(perm_smem);
-  constexpr int kBuf = tile_buf_elems((int)sizeof(T));
-  const int64_t per = (ntiles + gridDim.x - 1) / gridDim.x;
-  const int64_t t_begin = (int64_t)blockIdx.x * per, t_end = min(ntiles, t_begin + per);
-  if (t_begin >= t_end) return;
-  // the block owning the first work item; later items walk forward from it
-  int lo = 0, hi = nd - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (descs[mid].tile_begin <= t_begin) lo = mid; else hi = mid - 1;
-  }
-  // the current block's descriptor, staged in shared memory when the walk reaches a new block
-  __shared__ PermDesc sdesc;
-  int cur = -1;
-  int b = 0;              // the buffer of the current tile item
-  bool pending = false;   // its loads were issued by the previous item
-  // first work item of the next block, read from global memory only when the walk moves on
-  constexpr int64_t kNone = 0x7FFFFFFFFFFFFFFFll;
-  int64_t next_begin = lo + 1 < nd ? descs[lo + 1].tile_begin : kNone;
-  for (int64_t t = t_begin; t < t_end; ++t) {
-    while (t >= next_begin) {
-      ++lo;
-      next_begin = lo + 1 < nd ? descs[lo + 1].tile_begin : kNone;
+  constexpr int kCap = perm_cap((int)sizeof(T));
+  constexpr int kBatch = 8;   // loads in flight per lane of a copy
+  __shared__ __align__(16) T s_buf[kPermWarps][kCap];
+  const int warp = threadIdx.x >> 5;
+  const uint32_t lane = threadIdx.x & 31;
+  T* S = s_buf[warp];
+  const int64_t first = (int64_t)blockIdx.x * kPermWarps + warp, step = (int64_t)gridDim.x * kPermWarps;
+  int next = item_block && first < nitems ? __ldg(item_block + first) : 0;
+  for (int64_t item = first; item < nitems; item += step) {
+    int b = next;
+    if (item_block) {
+      // the next item's descriptor is on its way while this one is worked on
+      if (item + step < nitems) {
+        next = __ldg(item_block + item + step);
+        if (lane < (sizeof(PermDesc) + 127) / 128)
+          asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(descs + next) + min(lane * 128, (uint32_t)sizeof(PermDesc) - 1)));
+      }
+    } else {
+      int hi = nd - 1;
+      b = 0;
+      while (b < hi) {
+        const int mid = (b + hi + 1) >> 1;
+        if (descs[mid].tile_begin <= item) b = mid; else hi = mid - 1;
+      }
     }
-    if (lo != cur) {   // uniform across the CTA: every thread walks the same items
-      __syncthreads();
-      if (threadIdx.x == 0) sdesc = descs[lo];
-      __syncthreads();
-      cur = lo;
-    }
-    const PermDesc& d = sdesc;
-    const int64_t local = t - d.tile_begin;
-    const int r = d.rank;
-    const int q = r - 1;
+    const PermDesc& d = descs[b];
+    const uint32_t local = (uint32_t)(item - d.tile_begin);
     const uint64_t sg = d.sign_mask;
-    if (r == 0) {   // single element
-      if (threadIdx.x == 0) dst[d.dst_off] = flip(src[d.src_off], sg);
-      continue;
-    }
-    // Offsets inside a block are below 2^31 (checked on the host), so the index arithmetic
-    // below is 32-bit; destination strides are running products (no per-thread stride array,
-    // which kept the kernel at 128 registers).
-    if (d.p < 0) {
-      // gather mode (both inner dims short): 1024 consecutive destination elements per work
-      // item, each thread decodes its source offset; block sizes are below 2^31 (checked on
-      // the host), so the index arithmetic is 32-bit
-      const uint32_t total = (uint32_t)d.nouter;
-      const uint32_t e0 = (uint32_t)local * kRunChunk;
-      const uint32_t e1 = min(e0 + (uint32_t)kRunChunk, total);
-      for (uint32_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-        uint32_t rem = e, soff = 0;
-        for (int i = r - 1; i >= 0; --i) {
-          const uint32_t di = (uint32_t)d.dims[i];
-          const uint32_t qq = rem / di;
-          soff += (rem - qq * di) * (uint32_t)d.sstride[i];
-          rem = qq;
-        }
-        dst[d.dst_off + e] = flip(src[d.src_off + soff], sg);
-      }
-      continue;
-    }
-    if (d.p == q && d.tq > 1) {
-      // copy mode with short runs: a work item is d.tq consecutive runs (of dims[q] elements,
-      // contiguous on both sides). The runs' offsets are decoded once, one thread per run,
-      // into shared memory (the tile buffers are idle: only tile items prefetch into them);
-      // then the item's elements are copied as one flat range, kLoadBatch loads in flight
-      // per thread before the stores.
-      const uint32_t len = (uint32_t)d.dims[q];
-      const uint32_t nruns = (uint32_t)(d.nouter);
-      const uint32_t r0 = (uint32_t)local * (uint32_t)d.tq;
-      const uint32_t nr = min(nruns, r0 + (uint32_t)d.tq) - r0;
-      uint32_t* run_s = reinterpret_cast<uint32_t*>(perm_smem);
-      uint32_t* run_d = run_s + nr;
-      for (uint32_t j = threadIdx.x; j < nr; j += kPermThreads) {
-        uint32_t rem = r0 + j, soff = 0, doff = 0, dstr = len;
-        for (int i = r - 2; i >= 0; --i) {
-          const uint32_t di = (uint32_t)d.dims[i];
-          const uint32_t qq = rem / di;
-          const uint32_t x = rem - qq * di;
-          rem = qq;
-          soff += x * (uint32_t)d.sstride[i];
-          doff += x * dstr;
-          dstr *= di;
-        }
-        run_s[j] = soff;
-        run_d[j] = doff;
-      }
-      __syncthreads();
-      const uint32_t total = nr * len;
-      const float rlen = 1.0f / (float)len;
-      const T* s = src + d.src_off;
-      T* o = dst + d.dst_off;
-      for (uint32_t e0 = threadIdx.x; e0 < total; e0 += kPermThreads * kLoadBatch) {
-        T v[kLoadBatch];
-        uint32_t at[kLoadBatch];
-#pragma unroll
-        for (int i = 0; i < kLoadBatch; ++i) {
-          const uint32_t e = e0 + (uint32_t)i * kPermThreads;
-          if (e < total) {
-            // run = e / len: the float quotient, corrected to the exact one
-            uint32_t run = (uint32_t)((float)e * rlen);
-            if (run * len > e) --run;
-            else if ((run + 1) * len <= e) ++run;
-            const uint32_t off = e - run * len;
-            v[i] = __ldg(s + run_s[run] + off);
-            at[i] = run_d[run] + off;
+    const T* s = src + d.src_off;
+    T* o = dst + d.dst_off;
+    if (d.mode == kPermTile) {
+      // the tile's place: p0, p1, q0, q1 tiles, then the outer index
+      uint32_t rem = local, t0 = d.tp[0], t1 = d.tp[1], t2 = d.tq[0], t3 = d.tq[1];
+      uint32_t x = rem / t0;
+      const uint32_t p0 = (rem - x * t0) * d.ep[0];
+      rem = x; x = rem / t1;
+      const uint32_t p1 = (rem - x * t1) * d.ep[1];
+      rem = x; x = rem / t2;
+      const uint32_t q0 = (rem - x * t2) * d.eq[0];
+      rem = x; x = rem / t3;
+      const uint32_t q1 = (rem - x * t3) * d.eq[1];
+      uint32_t soff, doff;
+      outer_offsets(d, x, soff, doff);
+      const uint32_t wp0 = min(d.ep[0], d.np[0] - p0), wp1 = min(d.ep[1], d.np[1] - p1);
+      const uint32_t wq0 = min(d.eq[0], d.nq[0] - q0), wq1 = min(d.eq[1], d.nq[1] - q1);
+      const uint32_t wp = wp0 * wp1, wq = wq0 * wq1, n = wp * wq, pitch = wp | 1;
+      const uint32_t sq0 = d.sq[0], sq1 = d.sq[1], dp0 = d.dp[0], dp1 = d.dp[1];
+      // p1 (q1) tiles hold all of p0 (q0), so P (Q) is one contiguous range of the source (destination)
+      s += soff + p0 + p1 * d.np[0] + q0 * sq0 + q1 * sq1;
+      o += doff + q0 + q1 * d.nq[0] + p0 * dp0 + p1 * dp1;
+      // A side of 17 .. 32 goes one lane per index, the other side's offset carried along; any
+      // other extent as one flat range, divided by its extents.
+      if (wp > 16 && wp <= 32) {
+        if (lane < wp) {
+          const T* row = s + lane;
+          T* at = S + lane;
+          const uint32_t wrap = sq1 - wq0 * sq0;
+          uint32_t y0 = 0;
+#pragma unroll 8
+          for (uint32_t q = 0; q < wq; ++q) {
+            cp_async_elem(at, row);
+            at += pitch;
+            row += sq0;
+            if (++y0 == wq0) {
+              y0 = 0;
+              row += (int32_t)wrap;
+            }
           }
         }
-#pragma unroll
-        for (int i = 0; i < kLoadBatch; ++i) {
-          const uint32_t e = e0 + (uint32_t)i * kPermThreads;
-          if (e < total) o[at[i]] = flip(v[i], sg);
-        }
-      }
-      __syncthreads();   // the run tables are rewritten by the next item
-      continue;
-    }
-    if (d.p == q) {
-      // copy mode: innermost run of length dims[q] contiguous on both sides
-      const uint32_t chunks_per_run = ((uint32_t)d.dims[q] + kRunChunk - 1) / kRunChunk;
-      const uint32_t run = (uint32_t)local / chunks_per_run;
-      const int64_t c0 = (int64_t)((uint32_t)local - run * chunks_per_run) * kRunChunk;
-      uint32_t rem = run, soff = 0, doff = 0, dstr = (uint32_t)d.dims[q];
-      for (int i = r - 2; i >= 0; --i) {
-        const uint32_t di = (uint32_t)d.dims[i];
-        const uint32_t qq = rem / di;
-        const uint32_t x = rem - qq * di;
-        rem = qq;
-        soff += x * (uint32_t)d.sstride[i];
-        doff += x * dstr;
-        dstr *= di;
-      }
-      const T* s = src + d.src_off + soff;
-      T* o = dst + d.dst_off + doff;
-      const int64_t n = min((int64_t)kRunChunk, (int64_t)d.dims[q] - c0);
-      if (sizeof(T) == 8 && ((((uintptr_t)(s + c0)) | ((uintptr_t)(o + c0))) & 15) == 0) {
-        // 16-byte vectors, kLoadBatch loads in flight per thread before the stores
-        const int64_t n2 = n >> 1;
-        const double2* s2 = reinterpret_cast<const double2*>(s + c0);
-        double2* o2 = reinterpret_cast<double2*>(o + c0);
-        for (int64_t e0 = threadIdx.x; e0 < n2; e0 += (int64_t)blockDim.x * kLoadBatch) {
-          double2 v[kLoadBatch];
-#pragma unroll
-          for (int i = 0; i < kLoadBatch; ++i) {
-            const int64_t e = e0 + (int64_t)i * blockDim.x;
-            if (e < n2) v[i] = __ldg(s2 + e);
-          }
-#pragma unroll
-          for (int i = 0; i < kLoadBatch; ++i) {
-            const int64_t e = e0 + (int64_t)i * blockDim.x;
-            if (e < n2) o2[e] = flip(v[i], sg);
-          }
-        }
-        if ((n & 1) && threadIdx.x == 0) o[c0 + n - 1] = flip(s[c0 + n - 1], sg);
       } else {
-        for (int64_t e0 = threadIdx.x; e0 < n; e0 += (int64_t)blockDim.x * kLoadBatch) {
-          T v[kLoadBatch];
-#pragma unroll
-          for (int i = 0; i < kLoadBatch; ++i) {
-            const int64_t e = e0 + (int64_t)i * blockDim.x;
-            if (e < n) v[i] = __ldg(s + c0 + e);
-          }
-#pragma unroll
-          for (int i = 0; i < kLoadBatch; ++i) {
-            const int64_t e = e0 + (int64_t)i * blockDim.x;
-            if (e < n) o[c0 + e] = flip(v[i], sg);
-          }
+        const uint32_t iwp = inv_of(wp), iwq0 = inv_of(wq0);
+#pragma unroll 4
+        for (uint32_t e = lane; e < n; e += 32) {
+          const uint32_t q = div_by(e, iwp), p = e - q * wp, y1 = div_by(q, iwq0), y0 = q - y1 * wq0;
+          cp_async_elem(S + q * pitch + p, s + (y0 * sq0 + y1 * sq1 + p));
         }
       }
-      continue;
-    }
-    // tile mode
-    T* cb = bufs + b * kBuf;
-    const TileJob<T> j = tile_job<T>(d, local, src, dst);
-    if (!pending) tile_loads(j, cb);
-    cp_async_wait_all();
-    __syncthreads();
-    // the next item's tile goes into the other buffer while this one is written out
-    pending = false;
-    if (t + 1 < t_end) {
-      int ln = lo;
-      if (t + 1 >= next_begin) {
-        ++ln;
-        while (ln + 1 < nd && descs[ln + 1].tile_begin <= t + 1) ++ln;
+      cp_async_wait_all();
+      __syncwarp();
+      if (wq > 16 && wq <= 32) {
+        if (lane < wq) {
+          T* row = o + lane;
+          const T* at = S + lane * pitch;
+          const uint32_t wrap = dp1 - wp0 * dp0;
+          uint32_t x0 = 0;
+#pragma unroll 8
+          for (uint32_t p = 0; p < wp; ++p) {
+            *row = flip(at[p], sg);
+            row += dp0;
+            if (++x0 == wp0) {
+              x0 = 0;
+              row += (int32_t)wrap;
+            }
+          }
+        }
+      } else {
+        const uint32_t iwq = inv_of(wq), iwp0 = inv_of(wp0);
+#pragma unroll 4
+        for (uint32_t e = lane; e < n; e += 32) {
+          const uint32_t p = div_by(e, iwq), q = e - p * wq, x1 = div_by(p, iwp0), x0 = p - x1 * wp0;
+          o[x0 * dp0 + x1 * dp1 + q] = flip(S[q * pitch + p], sg);
+        }
       }
-      const PermDesc& dn = ln == lo ? sdesc : descs[ln];
-      if (is_tile_item(dn)) {
-        tile_loads(tile_job<T>(dn, t + 1 - dn.tile_begin, src, dst), bufs + (b ^ 1) * kBuf);
-        pending = true;
+    } else if (d.mode == kPermWhole) {
+      const uint32_t n = d.size;
+#pragma unroll 4
+      for (uint32_t e = lane; e < n; e += 32) cp_async_elem(S + e, s + e);
+      cp_async_wait_all();
+      __syncwarp();
+      for (uint32_t e = lane; e < n; e += 32) {
+        uint32_t rem = e, at = 0;
+        for (int i = d.nd - 1; i >= 0; --i) {
+          const uint32_t x = div_by(rem, d.dstr[i]);   // here the dims' reciprocals
+          at += (rem - x * d.dims[i]) * d.sstr[i];
+          rem = x;
+        }
+        o[e] = flip(S[at], sg);
+      }
+    } else if (d.per > 1) {
+      // runs run0 .. run0 + nr - 1, their offsets once (one lane per run) into the buffer
+      const uint32_t len = d.size, run0 = local * d.per;
+      uint32_t runs = 1;
+      for (int i = 0; i < d.nd; ++i) runs *= d.dims[i];
+      const uint32_t nr = min(d.per, runs - run0), n = nr * len, inv = inv_of(len);
+      uint2* off = reinterpret_cast<uint2*>(S);
+      for (uint32_t r = lane; r < nr; r += 32) outer_offsets(d, run0 + r, off[r].x, off[r].y);
+      __syncwarp();
+      for (uint32_t e0 = lane; e0 < n; e0 += 32 * kBatch) {
+        T v[kBatch];
+        uint32_t at[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          const uint32_t e = e0 + 32 * u;
+          if (e < n) {
+            const uint32_t r = div_by(e, inv), x = e - r * len;
+            const uint2 f = off[r];
+            v[u] = __ldg(s + (f.x + x));
+            at[u] = f.y + x;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+          if (e0 + 32 * u < n) o[at[u]] = flip(v[u], sg);
+      }
+    } else {
+      // a piece of a long run
+      const uint32_t len = d.size, chunk = (uint32_t)kCap & ~31u, pieces = (len + chunk - 1) / chunk, run = local / pieces;
+      const uint32_t c0 = (local - run * pieces) * chunk, n = min(chunk, len - c0);
+      uint32_t soff, doff;
+      outer_offsets(d, run, soff, doff);
+      s += soff + c0;
+      o += doff + c0;
+      for (uint32_t e0 = lane; e0 < n; e0 += 32 * kBatch) {
+        T v[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+          if (e0 + 32 * u < n) v[u] = __ldg(s + e0 + 32 * u);
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+          if (e0 + 32 * u < n) o[e0 + 32 * u] = flip(v[u], sg);
       }
     }
-    tile_stores(j, cb);
-    __syncthreads();
-    b ^= 1;
+    __syncwarp();   // the buffer is free again
   }
-  cp_async_wait_all();
 }
 
-// dynamic shared memory of k_permute (also set as the kernel's maximum, per device)
-size_t perm_smem_bytes(int elem_bytes) { return (size_t)2 * tile_buf_elems(elem_bytes) * elem_bytes; }
-
-// once per device (the attribute belongs to the current device's copy of the kernel)
-void perm_set_smem_attr() {
-  static std::mutex mu;
-  static bool done[64] = {};
-  int dev = 0;
-  QLTG_CUDA(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lock(mu);
-  if (dev >= 0 && dev < 64 && done[dev]) return;
-  QLTG_CUDA(cudaFuncSetAttribute(k_permute<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)perm_smem_bytes(8)));
-  QLTG_CUDA(cudaFuncSetAttribute(k_permute<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)perm_smem_bytes(16)));
-  if (dev >= 0 && dev < 64) done[dev] = true;
+// Items of one block; fills the descriptor's mode and shape from its squeezed dims in destination
+// order (extents dd, source strides ds, innermost last).
+int64_t plan_block(PermDesc& d, int m, const int64_t* dd, const int64_t* ds, int elem_bytes) {
+  const int cap = perm_cap(elem_bytes);
+  int64_t total = 1, dstr[kMaxRank];
+  for (int i = m - 1; i >= 0; --i) {
+    dstr[i] = total;
+    total *= dd[i];
+  }
+  auto keep = [&](int i) {   // dim i joins the descriptor's list
+    d.dims[d.nd] = (uint32_t)dd[i];
+    d.sstr[d.nd] = (uint32_t)ds[i];
+    d.dstr[d.nd] = (uint32_t)dstr[i];
+    ++d.nd;
+  };
+  int p = -1;
+  for (int i = 0; i < m; ++i)
+    if (ds[i] == 1) p = i;
+  if (m == 0 || p == m - 1) {
+    // runs; a small block is one flat item either way
+    d.mode = kPermRuns;
+    const int64_t len = m ? dd[m - 1] : 1, runs = total / len;
+    for (int i = 0; i < m - 1; ++i) keep(i);
+    d.size = (uint32_t)len;
+    if (2 * len <= cap && runs > 1) {
+      // as many runs as the buffer has room for their data; their offsets (8 bytes each) fit then too
+      d.per = (uint32_t)std::max<int64_t>(2, cap / len);
+      return (runs + d.per - 1) / d.per;
+    }
+    d.per = 1;
+    const int64_t chunk = cap & ~31;
+    return runs * ((len + chunk - 1) / chunk);
+  }
+  // tile: q0 = the innermost destination dim, p0 = the innermost source dim; a short one takes
+  // its neighbour as a second dim
+  constexpr int kShort = 16;
+  const int q0 = m - 1;
+  int q1 = -1, p1 = -1;
+  if (dd[q0] <= kShort && m - 2 != p) q1 = m - 2;
+  if (dd[p] <= kShort)
+    for (int i = 0; i < m; ++i)
+      if (ds[i] == dd[p] && i != q0 && i != q1) p1 = i;
+  const int side = elem_bytes == 16 ? 22 : 32;
+  int64_t np[2] = {dd[p], p1 >= 0 ? dd[p1] : 1}, nq[2] = {dd[q0], q1 >= 0 ? dd[q1] : 1}, ep[2], eq[2];
+  auto start = [&](const int64_t* n, int64_t* e, bool two) {
+    e[0] = two ? n[0] : std::min<int64_t>(n[0], side);
+    e[1] = two ? std::min<int64_t>(n[1], std::max<int64_t>(1, side / n[0])) : 1;
+  };
+  start(np, ep, p1 >= 0);
+  start(nq, eq, q1 >= 0);
+  // grow the side that can while the tile leaves half the buffer unused
+  auto fits = [&](int64_t a0, int64_t a1, int64_t b0, int64_t b1) { return ((a0 * a1) | 1) * b0 * b1 <= cap; };
+  for (bool grown = true; grown;) {
+    grown = false;
+    int64_t& gp = p1 >= 0 ? ep[1] : ep[0];
+    int64_t& gq = q1 >= 0 ? eq[1] : eq[0];
+    const int64_t lp = p1 >= 0 ? np[1] : np[0], lq = q1 >= 0 ? nq[1] : nq[0];
+    for (int side_no = 0; side_no < 2 && !grown; ++side_no) {
+      int64_t& g = side_no == 0 ? gp : gq;
+      const int64_t l = side_no == 0 ? lp : lq, was = g;
+      if (g >= l) continue;
+      g = std::min(l, 2 * g);
+      if (fits(ep[0], ep[1], eq[0], eq[1])) grown = true;
+      else g = was;
+    }
+  }
+  int64_t outer = total, tiles = 1;
+  for (int i = 0; i < 2; ++i) {
+    for (auto [n, e, t] : {std::tuple<int64_t*, int64_t*, uint32_t*>{&np[i], &ep[i], &d.tp[i]}, {&nq[i], &eq[i], &d.tq[i]}}) {
+      const int64_t cnt = (*n + *e - 1) / *e;
+      *e = (*n + cnt - 1) / cnt;   // even pieces
+      *t = (uint32_t)((*n + *e - 1) / *e);
+      tiles *= *t;
+      outer /= *n;
+    }
+    d.np[i] = (uint32_t)np[i];
+    d.ep[i] = (uint32_t)ep[i];
+    d.nq[i] = (uint32_t)nq[i];
+    d.eq[i] = (uint32_t)eq[i];
+  }
+  if (outer > 1 && total <= cap) {
+    d.mode = kPermWhole;
+    for (int i = 0; i < m; ++i) {
+      keep(i);
+      d.dstr[i] = inv_of((uint32_t)dd[i]);
+    }
+    d.size = (uint32_t)total;
+    return 1;
+  }
+  d.mode = kPermTile;
+  d.dp[0] = (uint32_t)dstr[p];
+  d.dp[1] = p1 >= 0 ? (uint32_t)dstr[p1] : 0;
+  d.sq[0] = (uint32_t)ds[q0];
+  d.sq[1] = q1 >= 0 ? (uint32_t)ds[q1] : 0;
+  for (int i = 0; i < m; ++i)
+    if (i != p && i != p1 && i != q0 && i != q1) keep(i);
+  return tiles * outer;
 }
 
-int pow2_at_least(int64_t x, int cap) {
-  int v = 1;
-  while (v < x && v < cap) v <<= 1;
-  return v;
+template <typename T>
+void launch_permute(const PermDesc* descs, int64_t nblocks, const int32_t* item_block, int64_t nitems, const void* src,
+                    void* dst, cudaStream_t s) {
+  const unsigned grid = (unsigned)std::min<int64_t>((nitems + kPermWarps - 1) / kPermWarps,
+                                                    (int64_t)current_sm_count() * kPermCtasPerSm);
+  k_permute<T><<<grid, kPermThreads, 0, s>>>(descs, (int)nblocks, item_block, nitems, static_cast<const T*>(src),
+                                             static_cast<T*>(dst));
+  QLTG_CUDA(cudaGetLastError());
 }
 
 }  // namespace
@@ -407,10 +351,10 @@ void TransposeList::describe(const Meta& t, const std::vector<int>& order, const
                              const std::vector<int64_t>* dst_offsets, bool skip_identity,
                              const std::vector<uint8_t>* skip) {
   host.clear();
+  host.reserve(t.nblk);
   identity.assign(t.nblk, 0);
   ntiles = 0;
   const int r = t.rank;
-  const int budget = tile_budget((int)t.elem_bytes());   // elements per tile (32 KB of data)
   for (int64_t b = 0; b < t.nblk; ++b) {
     PermDesc d{};
     d.src_off = t.offsets[b];
@@ -441,78 +385,12 @@ void TransposeList::describe(const Meta& t, const std::vector<int>& order, const
         ++m;
       }
     }
-    d.rank = m;
-    d.p = -1;
-    for (int i = 0; i < m; ++i) {
-      QLTG_CHECK(dd[i] < ((int64_t)1 << 31), QLTG_ERR_UNSUPPORTED, "block dimension above 2^31");
-      d.dims[i] = (int32_t)dd[i];
-      d.sstride[i] = ds[i];
-      if (ds[i] == 1) d.p = i;
-    }
+    for (int i = 0; i < m; ++i) QLTG_CHECK(dd[i] < ((int64_t)1 << 31), QLTG_ERR_UNSUPPORTED, "block dimension above 2^31");
     QLTG_CHECK(t.blk_size(b) < ((int64_t)1 << 31), QLTG_ERR_UNSUPPORTED, "block with 2^31 or more elements");
     // at most one non-unit dim left after merging: the block's data is laid out the same way
     identity[b] = m <= 1 && d.sign_mask == 0 && d.src_off == d.dst_off;
-    int64_t tiles;
-    if ((identity[b] && skip_identity) || (skip && (*skip)[b])) {
-      tiles = 0;
-    } else if (m == 0) {
-      d.p = 0;
-      tiles = 1;
-    } else if (d.p == m - 1) {
-      const int64_t runs = t.blk_size(b) / dd[m - 1];
-      if (dd[m - 1] * 2 <= kRunChunk) {
-        // short runs: several per work item (tq = runs per item)
-        d.tq = (int32_t)std::max<int64_t>(2, kRunChunk / dd[m - 1]);
-        d.nouter = runs;
-        tiles = (runs + d.tq - 1) / d.tq;
-      } else {
-        d.tq = 1;
-        tiles = runs * ((dd[m - 1] + kRunChunk - 1) / kRunChunk);
-      }
-    } else {
-      // tile extents: 32 x 32, or stretched along the longer dim when the other is short
-      int tp = -1, tq = -1;
-      if (d.p >= 0) {
-        const int a = pow2_at_least(dd[d.p], budget), c = pow2_at_least(dd[m - 1], budget);
-        if (a >= kTile && c >= kTile) {
-          tp = tq = kTile;
-        } else if (a < kTile) {
-          tp = a;
-          tq = std::min(c, budget / a);
-        } else {
-          tq = c;
-          tp = std::min(a, budget / c);
-        }
-      }
-      if (tp < 0 || tp * tq < 64) {
-        // both inner dims short: destination-ordered gather
-        d.p = -1;
-        d.nouter = t.blk_size(b);
-        tiles = (d.nouter + kRunChunk - 1) / kRunChunk;
-      } else {
-        d.tp = tp;
-        d.tq = tq;
-        d.tiles_p = (int32_t)((dd[d.p] + tp - 1) / tp);
-        d.tiles_q = (int32_t)((dd[m - 1] + tq - 1) / tq);
-        // batch the largest remaining dim when the (p, q) tile holds few valid elements
-        d.u = -1;
-        d.tu = 1;
-        const int64_t valid = std::min<int64_t>(dd[d.p], tp) * std::min<int64_t>(dd[m - 1], tq);
-        int64_t best = 1;
-        for (int i = 0; i < m - 1; ++i)
-          if (i != d.p && dd[i] > best) { best = dd[i]; d.u = i; }
-        if (d.u >= 0 && valid < budget / 2) {
-          int tu = 1;
-          while (tu * 2 <= budget / (tp * tq) && tu * 2 * valid <= budget && tu < dd[d.u]) tu *= 2;
-          d.tu = tu;
-        } else {
-          d.u = -1;
-        }
-        d.tiles_u = (int32_t)(d.u >= 0 ? (dd[d.u] + d.tu - 1) / d.tu : 1);
-        d.nouter = t.blk_size(b) / (dd[d.p] * dd[m - 1] * (d.u >= 0 ? dd[d.u] : 1));
-        tiles = d.nouter * d.tiles_p * d.tiles_q * d.tiles_u;
-      }
-    }
+    const bool none = (identity[b] && skip_identity) || (skip && (*skip)[b]);
+    const int64_t tiles = none ? 0 : plan_block(d, m, dd, ds, (int)t.elem_bytes());
     d.tile_begin = ntiles;
     ntiles += tiles;
     host.push_back(d);
@@ -524,20 +402,21 @@ void TransposeList::build(const Meta& t, const std::vector<int>& order, const st
                           const std::vector<int64_t>* dst_offsets, cudaStream_t s, bool skip_identity,
                           const std::vector<uint8_t>* skip) {
   describe(t, order, signs, dst_offsets, skip_identity, skip);
+  QLTG_CHECK(ntiles < ((int64_t)1 << 32) && nblocks < ((int64_t)1 << 31), QLTG_ERR_UNSUPPORTED, "permutation too large");
+  // the block of every item goes behind the descriptors: one allocation, one copy
+  host.resize(nblocks + (ntiles * sizeof(int32_t) + sizeof(PermDesc) - 1) / sizeof(PermDesc));
+  int32_t* item = reinterpret_cast<int32_t*>(host.data() + nblocks);
+  for (int64_t b = 0; b < nblocks; ++b)
+    std::fill(item + host[b].tile_begin, item + (b + 1 < nblocks ? host[b + 1].tile_begin : ntiles), (int32_t)b);
   dev = upload(host, s);
 }
 
 void TransposeList::launch(const void* src, void* dst, int elem_bytes, cudaStream_t s) const {
   if (ntiles == 0) return;
-  perm_set_smem_attr();
-  const unsigned grid = (unsigned)std::min<int64_t>(ntiles, (int64_t)current_sm_count() * 8);
-  if (elem_bytes == 8)
-    k_permute<double><<<grid, kPermThreads, perm_smem_bytes(8), s>>>(dev.as<PermDesc>(), (int)nblocks, ntiles, static_cast<const double*>(src),
-                                           static_cast<double*>(dst));
-  else
-    k_permute<double2><<<grid, kPermThreads, perm_smem_bytes(16), s>>>(dev.as<PermDesc>(), (int)nblocks, ntiles,
-                                            static_cast<const double2*>(src), static_cast<double2*>(dst));
-  QLTG_CUDA(cudaGetLastError());
+  const PermDesc* descs = dev.as<PermDesc>();
+  const int32_t* item = reinterpret_cast<const int32_t*>(descs + nblocks);
+  if (elem_bytes == 8) launch_permute<double>(descs, nblocks, item, ntiles, src, dst, s);
+  else launch_permute<double2>(descs, nblocks, item, ntiles, src, dst, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -546,7 +425,7 @@ void TransposeList::launch(const void* src, void* dst, int elem_bytes, cudaStrea
 // framework's pool (a cudaMalloc then fails or evicts that pool's cache), or a loop that
 // cannot pay for the device-wide synchronisation of cudaMalloc / cudaFree - so the per-call
 // permutation work list lives in this fixed device table instead of a fresh cudaMalloc.
-// Every GPU that loads the library holds the table (about 600 KB) until the process exits.
+// Every GPU that loads the library holds the table (about 850 KB) until the process exits.
 // All calls share it and it keeps the last call's descriptors, so calls that overlap on the
 // GPU (on different streams at once) race; each call waits for its own kernel before
 // returning. The table's device address is looked up once per device and kept for the life
@@ -575,17 +454,10 @@ void launch_permute_noalloc(int device, const TransposeList& tl, const void* src
              "qltg_transpose_noalloc: tensor has " + std::to_string(tl.nblocks) + " blocks, the fixed table holds " +
                  std::to_string(kNoAllocPermBlocks));
   PermDesc* table = noalloc_table(device);
-  perm_set_smem_attr();
   if (tl.ntiles == 0) return;
   QLTG_CUDA(cudaMemcpyAsync(table, tl.host.data(), tl.host.size() * sizeof(PermDesc), cudaMemcpyHostToDevice, s));
-  const unsigned grid = (unsigned)std::min<int64_t>(tl.ntiles, (int64_t)current_sm_count() * 8);
-  if (elem_bytes == 8)
-    k_permute<double><<<grid, kPermThreads, perm_smem_bytes(8), s>>>(table, (int)tl.nblocks, tl.ntiles, static_cast<const double*>(src),
-                                           static_cast<double*>(dst));
-  else
-    k_permute<double2><<<grid, kPermThreads, perm_smem_bytes(16), s>>>(table, (int)tl.nblocks, tl.ntiles, static_cast<const double2*>(src),
-                                            static_cast<double2*>(dst));
-  QLTG_CUDA(cudaGetLastError());
+  if (elem_bytes == 8) launch_permute<double>(table, tl.nblocks, nullptr, tl.ntiles, src, dst, s);
+  else launch_permute<double2>(table, tl.nblocks, nullptr, tl.ntiles, src, dst, s);
   // the descriptors were copied from this call's host memory and the table is shared:
   // finish before returning
   QLTG_CUDA(cudaStreamSynchronize(s));

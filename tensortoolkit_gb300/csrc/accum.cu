@@ -89,16 +89,8 @@ void build_contiguous(CtrctPlan& p, qltg_ctx* ctx, const qltg_tensor_desc* a, co
   p.a = meta_from_desc(a);
   p.b = meta_from_desc(b);
   contiguous_plan_axes(p, a0, b0, n);
-  cudaStream_t s;
-  QLTG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-  try {
-    plan_contraction(p, s);
-    finalize_plan(p, s);
-  } catch (...) {
-    cudaStreamDestroy(s);
-    throw;
-  }
-  QLTG_CUDA(cudaStreamDestroy(s));
+  plan_contraction(p, ctx->plan_stream);
+  finalize_plan(p, ctx->plan_stream);
 }
 
 }  // namespace
@@ -200,11 +192,8 @@ int qltg_accum_plan_create(qltg_ctx* ctx, const qltg_tensor_desc* a, const qltg_
       }
     }
     if (expanded) *expanded = h->expanded ? 1 : 0;
-    cudaStream_t s;
-    QLTG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    h->d_items = upload(h->items, s);
-    QLTG_CUDA(cudaStreamSynchronize(s));
-    QLTG_CUDA(cudaStreamDestroy(s));
+    h->d_items = upload(h->items, ctx->plan_stream);
+    QLTG_CUDA(cudaStreamSynchronize(ctx->plan_stream));
     h->t_buf.alloc(std::max<int64_t>(T.size, 1) * T.elem_bytes());
     *plan = h.release();
   });

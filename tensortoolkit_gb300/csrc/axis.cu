@@ -277,16 +277,8 @@ int qltg_axis_rank2_plan_create(qltg_ctx* ctx, const qltg_tensor_desc* t, const 
     QLTG_CUDA(cudaSetDevice(ctx->device));
     auto h = std::make_unique<qltg_axis_plan>();
     h->ctx = ctx;
-    cudaStream_t s;
-    QLTG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    try {
-      h->s1.build(ctx, meta_from_desc(t), meta_from_desc(op), axis, s);
-      QLTG_CUDA(cudaStreamSynchronize(s));
-    } catch (...) {
-      cudaStreamDestroy(s);
-      throw;
-    }
-    QLTG_CUDA(cudaStreamDestroy(s));
+    h->s1.build(ctx, meta_from_desc(t), meta_from_desc(op), axis, ctx->plan_stream);
+    QLTG_CUDA(cudaStreamSynchronize(ctx->plan_stream));
     *plan = h.release();
   });
 }
@@ -301,17 +293,9 @@ int qltg_axis_two_rank2_plan_create(qltg_ctx* ctx, const qltg_tensor_desc* t, co
     auto h = std::make_unique<qltg_axis_plan>();
     h->ctx = ctx;
     h->two = true;
-    cudaStream_t s;
-    QLTG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    try {
-      h->s1.build(ctx, meta_from_desc(t), meta_from_desc(op1), axis1, s);
-      h->s2.build(ctx, h->s1.out, meta_from_desc(op2), axis2, s);
-      QLTG_CUDA(cudaStreamSynchronize(s));
-    } catch (...) {
-      cudaStreamDestroy(s);
-      throw;
-    }
-    QLTG_CUDA(cudaStreamDestroy(s));
+    h->s1.build(ctx, meta_from_desc(t), meta_from_desc(op1), axis1, ctx->plan_stream);
+    h->s2.build(ctx, h->s1.out, meta_from_desc(op2), axis2, ctx->plan_stream);
+    QLTG_CUDA(cudaStreamSynchronize(ctx->plan_stream));
     h->mid.alloc(std::max<int64_t>(h->s1.out.size, 1) * h->s1.out.elem_bytes());
     *plan = h.release();
   });
@@ -410,12 +394,9 @@ int qltg_axis_monomial_plan_create(qltg_ctx* ctx, const qltg_tensor_desc* t, int
         maps.insert(maps.end(), v.begin(), v.end());
       }
     }
-    cudaStream_t s;
-    QLTG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    h->d_mono_items = upload(items, s);
-    h->d_mono_maps = upload(maps, s);
-    QLTG_CUDA(cudaStreamSynchronize(s));
-    QLTG_CUDA(cudaStreamDestroy(s));
+    h->d_mono_items = upload(items, ctx->plan_stream);
+    h->d_mono_maps = upload(maps, ctx->plan_stream);
+    QLTG_CUDA(cudaStreamSynchronize(ctx->plan_stream));
     h->mono_items = (int)items.size();
     *plan = h.release();
   });

@@ -151,14 +151,16 @@ int qltg_create(int device, qltg_ctx** ctx) {
     QLTG_CUDA(cudaGetDeviceCount(&n));
     QLTG_CHECK(device >= 0 && device < n, QLTG_ERR_INVALID, "no such CUDA device");
     QLTG_CUDA(cudaSetDevice(device));
-    auto* c = new qltg_ctx;
+    auto c = std::make_unique<qltg_ctx>();
     c->device = device;
     cudaDeviceProp prop;
     QLTG_CUDA(cudaGetDeviceProperties(&prop, device));
     c->num_sms = prop.multiProcessorCount;
     c->cc_major = prop.major;
     c->cc_minor = prop.minor;
-    *ctx = c;
+    QLTG_CUDA(cudaStreamCreateWithFlags(&c->plan_stream, cudaStreamNonBlocking));
+    c->small_piece.alloc(256);
+    *ctx = c.release();
   });
 }
 
@@ -181,16 +183,8 @@ int qltg_ctrct_plan_create(qltg_ctx* ctx, const qltg_tensor_desc* a, const qltg_
     p.b = meta_from_desc(b);
     p.axa.assign(axes_a, axes_a + naxes);
     p.axb.assign(axes_b, axes_b + naxes);
-    cudaStream_t s;
-    QLTG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    try {
-      plan_contraction(p, s);
-      finalize_plan(p, s);
-    } catch (...) {
-      cudaStreamDestroy(s);
-      throw;
-    }
-    QLTG_CUDA(cudaStreamDestroy(s));
+    plan_contraction(p, ctx->plan_stream);
+    finalize_plan(p, ctx->plan_stream);
     *plan = h.release();
   });
 }

@@ -98,6 +98,7 @@ struct GemmSchedule {
   int64_t ntiles = 0;                   // tiles of all runs
   bool share_tiles = false;             // a CTA's warps share each tile (few or very long tiles)
   std::vector<GemmRowChunk> skinny;     // row chunks of skinny blocks (n, k <= 8)
+  DevBuf lists;                          // holds the device copies below (parts of it)
   DevBuf d_cblk, d_task, d_run, d_skinny, d_counter;
   int bm = 32;                          // rows of the FP64 tiles of a CTA's four warps
   int skinny_maxn = 8;                  // largest n of the skinny blocks (kernel variant)

@@ -1,6 +1,7 @@
 // Contraction execution: schedule construction after device pairing, and the launch
 // sequence (operand transposes, then one grouped GEMM).
 #include <algorithm>
+#include <cstring>
 
 #include "ctrct.h"
 #include "split.h"
@@ -154,14 +155,30 @@ void finalize_plan(CtrctPlan& p, cudaStream_t s) {
     if (p.b_tl.ntiles) p.b_t.alloc(p.b.size * eb);
   }
   if (!g.skinny.empty()) (void)skinny_grid((int)g.skinny.size(), p.a.dtype == QLTG_C128, g.skinny_maxn, p.ctx->num_sms);
-  g.d_cblk = upload(g.cblk, s);
-  g.d_task = upload(g.task, s);
-  g.d_run = upload(g.run, s);
-  g.d_skinny = upload(g.skinny, s);
-  g.d_counter.alloc(sizeof(int));
+  // the schedule's lists in one buffer, with one copy
+  {
+    const struct { const void* src; size_t bytes; DevBuf* part; } lists[] = {
+        {g.cblk.data(), g.cblk.size() * sizeof(GemmCBlk), &g.d_cblk},
+        {g.task.data(), g.task.size() * sizeof(GemmTask), &g.d_task},
+        {g.run.data(), g.run.size() * sizeof(GemmTileRun), &g.d_run},
+        {g.skinny.data(), g.skinny.size() * sizeof(GemmRowChunk), &g.d_skinny},
+        {nullptr, sizeof(int), &g.d_counter}};
+    auto room = [](size_t n) { return (n + 255) / 256 * 256; };
+    size_t total = 0;
+    for (const auto& l : lists) total += room(l.bytes);
+    std::vector<char> image(total, 0);
+    g.lists.alloc(total);
+    size_t at = 0;
+    for (const auto& l : lists) {
+      if (l.src) std::memcpy(image.data() + at, l.src, l.bytes);
+      *l.part = DevBuf::part(g.lists, at, l.bytes);
+      at += room(l.bytes);
+    }
+    QLTG_CUDA(cudaMemcpyAsync(g.lists.get(), image.data(), total, cudaMemcpyHostToDevice, s));
+    QLTG_CUDA(cudaStreamSynchronize(s));   // before the image goes, and before any stream uses the lists
+  }
   p.launches_per_exec = (g.ntiles ? 2 : 0) + (g.skinny.empty() ? 0 : 1) +   // memset + GEMM
                          (p.a_tl.ntiles ? 1 : 0) + (p.b_tl.ntiles ? 1 : 0);
-  QLTG_CUDA(cudaStreamSynchronize(s));
 }
 
 // Kernel launches of one split-mode execution: operand transposes plus the split stage.

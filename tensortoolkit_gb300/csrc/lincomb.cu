@@ -182,12 +182,9 @@ int qltg_lincomb_plan_create(qltg_ctx* ctx, int32_t n, const qltg_tensor_desc* c
     }
     QLTG_CHECK(h->items.size() < ((size_t)1 << 31) && h->srcs.size() < ((size_t)1 << 31), QLTG_ERR_UNSUPPORTED,
                "linear combination too large");
-    cudaStream_t s;
-    QLTG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    h->d_items = upload(h->items, s);
-    h->d_srcs = upload(h->srcs, s);
-    QLTG_CUDA(cudaStreamSynchronize(s));
-    QLTG_CUDA(cudaStreamDestroy(s));
+    h->d_items = upload(h->items, ctx->plan_stream);
+    h->d_srcs = upload(h->srcs, ctx->plan_stream);
+    QLTG_CUDA(cudaStreamSynchronize(ctx->plan_stream));
     *plan = h.release();
   });
 }

@@ -199,6 +199,187 @@ std::vector<T> download(const DevBuf& b, int64_t n, cudaStream_t s) {
   return v;
 }
 
+// The block pairs of a contraction and their output blocks: per pair in generation order (A blocks
+// outer, B blocks inner, both ascending) its A and B block, output block index and sign; per
+// output block, ascending, its index, first place in `perm` (the pairs sorted by output block,
+// stably) and element offset; m, k of every A block and n of every B block.
+struct Pairing {
+  std::vector<int32_t> a, b, sign, perm, c_first;
+  std::vector<uint64_t> cidx, c_idx;
+  std::vector<int64_t> c_off, m, k, n;
+};
+
+// Small plans are paired on the host: the device form's dozen launches, three waits and thirty
+// allocations take half a millisecond whatever the size (whole plan creation, 24 pairs: 672 us on
+// the device, 89 us here; 1196 bosonic pairs 974 / 380 us; 3396 fermionic ones 1245 / 712 us). The
+// line keeps what a plan past it wastes on counting here below 0.2 ms.
+constexpr int64_t kHostBlocks = 4096, kHostPairs = 4096;
+
+// False (nothing decided) when there are more than kHostPairs pairs.
+bool pair_on_host(const Meta& A, const Meta& B, const PairParams& P, const std::vector<int64_t>& dims_a,
+                  const std::vector<int64_t>& dims_b, const std::vector<uint8_t>& par_a,
+                  const std::vector<uint8_t>& par_b, Pairing& out) {
+  const int64_t na = A.nblk, nb = B.nblk;
+  std::vector<uint64_t> key_a(na);
+  std::vector<std::pair<uint64_t, int32_t>> key_b(nb);   // sorted by key, then block
+  out.m.resize(na);
+  out.k.resize(na);
+  out.n.resize(nb);
+  for (int64_t i = 0; i < na; ++i) {
+    const int64_t* c = &A.coords[i * P.ra];
+    uint64_t key = 0;
+    int64_t k = 1, m = 1;
+    for (int t = 0; t < P.nax; ++t) {
+      key += (uint64_t)c[P.axa[t]] * (uint64_t)P.key_w[t];
+      k *= dims_a[P.a_leg_off[P.axa[t]] + c[P.axa[t]]];
+    }
+    for (int t = 0; t < P.nsa; ++t) m *= dims_a[P.a_leg_off[P.sa[t]] + c[P.sa[t]]];
+    key_a[i] = key;
+    out.k[i] = k;
+    out.m[i] = m;
+  }
+  for (int64_t j = 0; j < nb; ++j) {
+    const int64_t* c = &B.coords[j * P.rb];
+    uint64_t key = 0;
+    int64_t n = 1;
+    for (int t = 0; t < P.nax; ++t) key += (uint64_t)c[P.axb[t]] * (uint64_t)P.key_w[t];
+    for (int t = 0; t < P.nsb; ++t) n *= dims_b[P.b_leg_off[P.sb[t]] + c[P.sb[t]]];
+    key_b[j] = {key, (int32_t)j};
+    out.n[j] = n;
+  }
+  std::sort(key_b.begin(), key_b.end());
+  std::vector<std::pair<uint64_t, int32_t>> by_c;   // (output block, pair): sorting keeps generation order
+  for (int64_t i = 0; i < na; ++i) {
+    const int64_t* c1 = &A.coords[i * P.ra];
+    uint64_t base = 0;
+    for (int t = 0; t < P.nsa; ++t) base += (uint64_t)c1[P.sa[t]] * (uint64_t)P.c_w[t];
+    uint8_t pa[kMaxRank], pb[kMaxRank];
+    if (P.fermionic)
+      for (int l = 0; l < P.ra; ++l) pa[l] = par_a[P.a_leg_off[l] + c1[l]];
+    for (auto it = std::lower_bound(key_b.begin(), key_b.end(), std::make_pair(key_a[i], (int32_t)-1));
+         it != key_b.end() && it->first == key_a[i]; ++it) {
+      if ((int64_t)out.a.size() == kHostPairs) {
+        out = Pairing();
+        return false;
+      }
+      const int64_t* c2 = &B.coords[(int64_t)it->second * P.rb];
+      uint64_t ci = base;
+      for (int u = 0; u < P.nsb; ++u) ci += (uint64_t)c2[P.sb[u]] * (uint64_t)P.c_w[P.nsa + u];
+      int sign = 1;
+      if (P.fermionic) {
+        for (int l = 0; l < P.rb; ++l) pb[l] = par_b[P.b_leg_off[l] + c2[l]];
+        sign = exchange_sign(pa, P.ra, pb, P.rb, P.sgn_axa, P.sgn_axb, P.nax, P.a_ctrct_in) *
+               saved_order_sign(pa, P.sa, P.nsa) * saved_order_sign(pb, P.sb, P.nsb);
+      }
+      by_c.push_back({ci, (int32_t)out.a.size()});
+      out.a.push_back((int32_t)i);
+      out.b.push_back(it->second);
+      out.cidx.push_back(ci);
+      out.sign.push_back(sign);
+    }
+  }
+  std::sort(by_c.begin(), by_c.end());
+  int64_t off = 0;
+  for (size_t q = 0; q < by_c.size(); ++q) {
+    const int32_t t = by_c[q].second;
+    out.perm.push_back(t);
+    if (q && by_c[q].first == by_c[q - 1].first) continue;
+    out.c_idx.push_back(by_c[q].first);
+    out.c_first.push_back((int32_t)q);
+    out.c_off.push_back(off);
+    off += out.m[out.a[t]] * out.n[out.b[t]];
+  }
+  return true;
+}
+
+void pair_on_device(const std::vector<int32_t>& ca, const std::vector<int32_t>& cb, const PairParams& P, const Meta& C,
+                    const std::vector<int64_t>& dims_a, const std::vector<int64_t>& dims_b,
+                    const std::vector<uint8_t>& par_a, const std::vector<uint8_t>& par_b, uint64_t key_count,
+                    cudaStream_t s, Pairing& out) {
+  const int64_t na = (int64_t)(ca.size() / P.ra), nb = (int64_t)(cb.size() / P.rb);
+  DevBuf d_ca = upload(ca, s), d_cb = upload(cb, s);
+  DevBuf d_da = upload(dims_a, s), d_db = upload(dims_b, s);
+  DevBuf d_pa = upload(par_a, s), d_pb = upload(par_b, s);
+  DevBuf d_keya(na * 8), d_ma(na * 8), d_ka(na * 8);
+  DevBuf d_keyb(nb * 8), d_keyb_s(nb * 8), d_nb(nb * 8), d_iotab(nb * 4), d_iotab_s(nb * 4);
+  k_keys_a<<<grid_for(na), 256, 0, s>>>(d_ca.as<int32_t>(), na, d_da.as<int64_t>(), P, d_keya.as<uint64_t>(),
+                                        d_ma.as<int64_t>(), d_ka.as<int64_t>());
+  k_keys_b<<<grid_for(nb), 256, 0, s>>>(d_cb.as<int32_t>(), nb, d_db.as<int64_t>(), P, d_keyb.as<uint64_t>(),
+                                        d_nb.as<int64_t>(), d_iotab.as<int32_t>());
+  QLTG_CUDA(cudaGetLastError());
+  const int kbits = bits_for(key_count);
+  size_t tmp_bytes = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, d_keyb.as<uint64_t>(), d_keyb_s.as<uint64_t>(),
+                                  d_iotab.as<int32_t>(), d_iotab_s.as<int32_t>(), (int)nb, 0, kbits, s);
+  DevBuf d_tmp(std::max<size_t>(tmp_bytes, 16));
+  QLTG_CUDA(cub::DeviceRadixSort::SortPairs(d_tmp.get(), tmp_bytes, d_keyb.as<uint64_t>(), d_keyb_s.as<uint64_t>(),
+                                            d_iotab.as<int32_t>(), d_iotab_s.as<int32_t>(), (int)nb, 0, kbits, s));
+  DevBuf d_lo(na * 8), d_cnt(na * 8), d_off(na * 8);
+  k_match<<<grid_for(na), 256, 0, s>>>(d_keya.as<uint64_t>(), na, d_keyb_s.as<uint64_t>(), nb, d_lo.as<int64_t>(),
+                                       d_cnt.as<int64_t>());
+  QLTG_CUDA(cudaGetLastError());
+  tmp_bytes = 0;
+  cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, d_cnt.as<int64_t>(), d_off.as<int64_t>(), (int)na, s);
+  if (tmp_bytes > d_tmp.bytes()) d_tmp.alloc(tmp_bytes);
+  QLTG_CUDA(cub::DeviceScan::ExclusiveSum(d_tmp.get(), tmp_bytes, d_cnt.as<int64_t>(), d_off.as<int64_t>(), (int)na, s));
+  int64_t last_off = 0, last_cnt = 0;
+  QLTG_CUDA(cudaMemcpyAsync(&last_off, d_off.as<int64_t>() + na - 1, 8, cudaMemcpyDeviceToHost, s));
+  QLTG_CUDA(cudaMemcpyAsync(&last_cnt, d_cnt.as<int64_t>() + na - 1, 8, cudaMemcpyDeviceToHost, s));
+  QLTG_CUDA(cudaStreamSynchronize(s));
+  const int64_t np = last_off + last_cnt;
+  QLTG_CHECK(np < (int64_t)1 << 31, QLTG_ERR_UNSUPPORTED, "more than 2^31 block pairs");
+  if (np == 0) return;
+  DevBuf d_ppa(np * 4), d_ppb(np * 4), d_cidx(np * 8), d_cidx_s(np * 8), d_sign(np * 4), d_iota(np * 4), d_perm(np * 4);
+  k_emit<<<grid_for(na, 128), 128, 0, s>>>(d_ca.as<int32_t>(), d_cb.as<int32_t>(), na, d_lo.as<int64_t>(),
+                                           d_off.as<int64_t>(), d_cnt.as<int64_t>(), d_iotab_s.as<int32_t>(),
+                                           d_pa.as<uint8_t>(), d_pb.as<uint8_t>(), P, d_ppa.as<int32_t>(),
+                                           d_ppb.as<int32_t>(), d_cidx.as<uint64_t>(), d_sign.as<int32_t>(),
+                                           d_iota.as<int32_t>());
+  QLTG_CUDA(cudaGetLastError());
+  uint64_t cmax = 1;
+  for (int l = 0; l < P.rc; ++l) cmax *= (uint64_t)C.nsct(l);
+  const int cbits = bits_for(cmax);
+  tmp_bytes = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, d_cidx.as<uint64_t>(), d_cidx_s.as<uint64_t>(),
+                                  d_iota.as<int32_t>(), d_perm.as<int32_t>(), (int)np, 0, cbits, s);
+  if (tmp_bytes > d_tmp.bytes()) d_tmp.alloc(tmp_bytes);
+  QLTG_CUDA(cub::DeviceRadixSort::SortPairs(d_tmp.get(), tmp_bytes, d_cidx.as<uint64_t>(), d_cidx_s.as<uint64_t>(),
+                                            d_iota.as<int32_t>(), d_perm.as<int32_t>(), (int)np, 0, cbits, s));
+  DevBuf d_head(np * 4), d_cbi(np * 4);
+  k_heads<<<grid_for(np), 256, 0, s>>>(d_cidx_s.as<uint64_t>(), np, d_head.as<int32_t>());
+  QLTG_CUDA(cudaGetLastError());
+  tmp_bytes = 0;
+  cub::DeviceScan::InclusiveSum(nullptr, tmp_bytes, d_head.as<int32_t>(), d_cbi.as<int32_t>(), (int)np, s);
+  if (tmp_bytes > d_tmp.bytes()) d_tmp.alloc(tmp_bytes);
+  QLTG_CUDA(cub::DeviceScan::InclusiveSum(d_tmp.get(), tmp_bytes, d_head.as<int32_t>(), d_cbi.as<int32_t>(), (int)np, s));
+  int32_t ncb = 0;
+  QLTG_CUDA(cudaMemcpyAsync(&ncb, d_cbi.as<int32_t>() + np - 1, 4, cudaMemcpyDeviceToHost, s));
+  QLTG_CUDA(cudaStreamSynchronize(s));
+  DevBuf d_cidxu(ncb * 8), d_cfirst(ncb * 4), d_csize(ncb * 8), d_coff(ncb * 8);
+  k_cblocks<<<grid_for(np), 256, 0, s>>>(d_head.as<int32_t>(), d_cbi.as<int32_t>(), np, d_cidx_s.as<uint64_t>(),
+                                         d_perm.as<int32_t>(), d_ppa.as<int32_t>(), d_ppb.as<int32_t>(),
+                                         d_ma.as<int64_t>(), d_nb.as<int64_t>(), d_cidxu.as<uint64_t>(),
+                                         d_cfirst.as<int32_t>(), d_csize.as<int64_t>());
+  QLTG_CUDA(cudaGetLastError());
+  tmp_bytes = 0;
+  cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, d_csize.as<int64_t>(), d_coff.as<int64_t>(), ncb, s);
+  if (tmp_bytes > d_tmp.bytes()) d_tmp.alloc(tmp_bytes);
+  QLTG_CUDA(cub::DeviceScan::ExclusiveSum(d_tmp.get(), tmp_bytes, d_csize.as<int64_t>(), d_coff.as<int64_t>(), ncb, s));
+
+  out.c_idx = download<uint64_t>(d_cidxu, ncb, s);
+  out.c_first = download<int32_t>(d_cfirst, ncb, s);
+  out.c_off = download<int64_t>(d_coff, ncb, s);
+  out.perm = download<int32_t>(d_perm, np, s);
+  out.a = download<int32_t>(d_ppa, np, s);
+  out.b = download<int32_t>(d_ppb, np, s);
+  out.sign = download<int32_t>(d_sign, np, s);
+  out.cidx = download<uint64_t>(d_cidx, np, s);
+  out.m = download<int64_t>(d_ma, na, s);
+  out.k = download<int64_t>(d_ka, na, s);
+  out.n = download<int64_t>(d_nb, nb, s);
+  QLTG_CUDA(cudaStreamSynchronize(s));
+}
+
 }  // namespace
 
 int host_exchange_sign(const bool* pa, int ra, const bool* pb, int rb, const int64_t* axa, const int64_t* axb,
@@ -338,6 +519,8 @@ void plan_contraction(CtrctPlan& p, cudaStream_t s) {
     for (int64_t s2 = 0; s2 < B.nsct(l); ++s2) { dims_b.push_back(B.dims[l][s2]); par_b.push_back(B.parity(l, s2)); }
   }
   std::vector<int32_t> ca(A.coords.begin(), A.coords.end()), cb(B.coords.begin(), B.coords.end());
+  uint64_t key_count = 1;
+  for (int t = 0; t < nax; ++t) key_count *= (uint64_t)A.nsct((int)p.axa[t]);
 
   const int64_t na = A.nblk, nb = B.nblk;
   p.tasks_gen.clear();
@@ -349,93 +532,19 @@ void plan_contraction(CtrctPlan& p, cudaStream_t s) {
     return;
   }
 
-  DevBuf d_ca = upload(ca, s), d_cb = upload(cb, s);
-  DevBuf d_da = upload(dims_a, s), d_db = upload(dims_b, s);
-  DevBuf d_pa = upload(par_a, s), d_pb = upload(par_b, s);
-  DevBuf d_keya(na * 8), d_ma(na * 8), d_ka(na * 8);
-  DevBuf d_keyb(nb * 8), d_keyb_s(nb * 8), d_nb(nb * 8), d_iotab(nb * 4), d_iotab_s(nb * 4);
-  k_keys_a<<<grid_for(na), 256, 0, s>>>(d_ca.as<int32_t>(), na, d_da.as<int64_t>(), P, d_keya.as<uint64_t>(),
-                                        d_ma.as<int64_t>(), d_ka.as<int64_t>());
-  k_keys_b<<<grid_for(nb), 256, 0, s>>>(d_cb.as<int32_t>(), nb, d_db.as<int64_t>(), P, d_keyb.as<uint64_t>(),
-                                        d_nb.as<int64_t>(), d_iotab.as<int32_t>());
-  QLTG_CUDA(cudaGetLastError());
-  uint64_t kmax = 1;
-  for (int t = 0; t < nax; ++t) kmax *= (uint64_t)A.nsct((int)p.axa[t]);
-  const int kbits = bits_for(kmax);
-  size_t tmp_bytes = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, d_keyb.as<uint64_t>(), d_keyb_s.as<uint64_t>(),
-                                  d_iotab.as<int32_t>(), d_iotab_s.as<int32_t>(), (int)nb, 0, kbits, s);
-  DevBuf d_tmp(std::max<size_t>(tmp_bytes, 16));
-  QLTG_CUDA(cub::DeviceRadixSort::SortPairs(d_tmp.get(), tmp_bytes, d_keyb.as<uint64_t>(), d_keyb_s.as<uint64_t>(),
-                                            d_iotab.as<int32_t>(), d_iotab_s.as<int32_t>(), (int)nb, 0, kbits, s));
-  DevBuf d_lo(na * 8), d_cnt(na * 8), d_off(na * 8);
-  k_match<<<grid_for(na), 256, 0, s>>>(d_keya.as<uint64_t>(), na, d_keyb_s.as<uint64_t>(), nb, d_lo.as<int64_t>(),
-                                       d_cnt.as<int64_t>());
-  QLTG_CUDA(cudaGetLastError());
-  tmp_bytes = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, d_cnt.as<int64_t>(), d_off.as<int64_t>(), (int)na, s);
-  if (tmp_bytes > d_tmp.bytes()) d_tmp.alloc(tmp_bytes);
-  QLTG_CUDA(cub::DeviceScan::ExclusiveSum(d_tmp.get(), tmp_bytes, d_cnt.as<int64_t>(), d_off.as<int64_t>(), (int)na, s));
-  int64_t last_off = 0, last_cnt = 0;
-  QLTG_CUDA(cudaMemcpyAsync(&last_off, d_off.as<int64_t>() + na - 1, 8, cudaMemcpyDeviceToHost, s));
-  QLTG_CUDA(cudaMemcpyAsync(&last_cnt, d_cnt.as<int64_t>() + na - 1, 8, cudaMemcpyDeviceToHost, s));
-  QLTG_CUDA(cudaStreamSynchronize(s));
-  const int64_t np = last_off + last_cnt;
-  QLTG_CHECK(np < (int64_t)1 << 31, QLTG_ERR_UNSUPPORTED, "more than 2^31 block pairs");
+  Pairing pr;
+  if (na + nb > kHostBlocks || !pair_on_host(A, B, P, dims_a, dims_b, par_a, par_b, pr))
+    pair_on_device(ca, cb, P, C, dims_a, dims_b, par_a, par_b, key_count, s, pr);
+  const int64_t np = (int64_t)pr.a.size();
+  const int32_t ncb = (int32_t)pr.c_idx.size();
   if (np == 0) {
     C.nblk = 0;
     C.refresh_offsets();
     return;
   }
-  DevBuf d_ppa(np * 4), d_ppb(np * 4), d_cidx(np * 8), d_cidx_s(np * 8), d_sign(np * 4), d_iota(np * 4), d_perm(np * 4);
-  k_emit<<<grid_for(na, 128), 128, 0, s>>>(d_ca.as<int32_t>(), d_cb.as<int32_t>(), na, d_lo.as<int64_t>(),
-                                           d_off.as<int64_t>(), d_cnt.as<int64_t>(), d_iotab_s.as<int32_t>(),
-                                           d_pa.as<uint8_t>(), d_pb.as<uint8_t>(), P, d_ppa.as<int32_t>(),
-                                           d_ppb.as<int32_t>(), d_cidx.as<uint64_t>(), d_sign.as<int32_t>(),
-                                           d_iota.as<int32_t>());
-  QLTG_CUDA(cudaGetLastError());
-  uint64_t cmax = 1;
-  for (int l = 0; l < rc; ++l) cmax *= (uint64_t)C.nsct(l);
-  const int cbits = bits_for(cmax);
-  tmp_bytes = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, d_cidx.as<uint64_t>(), d_cidx_s.as<uint64_t>(),
-                                  d_iota.as<int32_t>(), d_perm.as<int32_t>(), (int)np, 0, cbits, s);
-  if (tmp_bytes > d_tmp.bytes()) d_tmp.alloc(tmp_bytes);
-  QLTG_CUDA(cub::DeviceRadixSort::SortPairs(d_tmp.get(), tmp_bytes, d_cidx.as<uint64_t>(), d_cidx_s.as<uint64_t>(),
-                                            d_iota.as<int32_t>(), d_perm.as<int32_t>(), (int)np, 0, cbits, s));
-  DevBuf d_head(np * 4), d_cbi(np * 4);
-  k_heads<<<grid_for(np), 256, 0, s>>>(d_cidx_s.as<uint64_t>(), np, d_head.as<int32_t>());
-  QLTG_CUDA(cudaGetLastError());
-  tmp_bytes = 0;
-  cub::DeviceScan::InclusiveSum(nullptr, tmp_bytes, d_head.as<int32_t>(), d_cbi.as<int32_t>(), (int)np, s);
-  if (tmp_bytes > d_tmp.bytes()) d_tmp.alloc(tmp_bytes);
-  QLTG_CUDA(cub::DeviceScan::InclusiveSum(d_tmp.get(), tmp_bytes, d_head.as<int32_t>(), d_cbi.as<int32_t>(), (int)np, s));
-  int32_t ncb = 0;
-  QLTG_CUDA(cudaMemcpyAsync(&ncb, d_cbi.as<int32_t>() + np - 1, 4, cudaMemcpyDeviceToHost, s));
-  QLTG_CUDA(cudaStreamSynchronize(s));
-  DevBuf d_cidxu(ncb * 8), d_cfirst(ncb * 4), d_csize(ncb * 8), d_coff(ncb * 8);
-  k_cblocks<<<grid_for(np), 256, 0, s>>>(d_head.as<int32_t>(), d_cbi.as<int32_t>(), np, d_cidx_s.as<uint64_t>(),
-                                         d_perm.as<int32_t>(), d_ppa.as<int32_t>(), d_ppb.as<int32_t>(),
-                                         d_ma.as<int64_t>(), d_nb.as<int64_t>(), d_cidxu.as<uint64_t>(),
-                                         d_cfirst.as<int32_t>(), d_csize.as<int64_t>());
-  QLTG_CUDA(cudaGetLastError());
-  tmp_bytes = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, d_csize.as<int64_t>(), d_coff.as<int64_t>(), ncb, s);
-  if (tmp_bytes > d_tmp.bytes()) d_tmp.alloc(tmp_bytes);
-  QLTG_CUDA(cub::DeviceScan::ExclusiveSum(d_tmp.get(), tmp_bytes, d_csize.as<int64_t>(), d_coff.as<int64_t>(), ncb, s));
-
-  auto h_cidxu = download<uint64_t>(d_cidxu, ncb, s);
-  auto h_cfirst = download<int32_t>(d_cfirst, ncb, s);
-  auto h_coff = download<int64_t>(d_coff, ncb, s);
-  auto h_perm = download<int32_t>(d_perm, np, s);
-  auto h_ppa = download<int32_t>(d_ppa, np, s);
-  auto h_ppb = download<int32_t>(d_ppb, np, s);
-  auto h_sign = download<int32_t>(d_sign, np, s);
-  auto h_cidx = download<uint64_t>(d_cidx, np, s);
-  auto h_ma = download<int64_t>(d_ma, na, s);
-  auto h_ka = download<int64_t>(d_ka, na, s);
-  auto h_nb = download<int64_t>(d_nb, nb, s);
-  QLTG_CUDA(cudaStreamSynchronize(s));
+  const auto &h_cidxu = pr.c_idx, &h_cidx = pr.cidx;
+  const auto &h_cfirst = pr.c_first, &h_perm = pr.perm, &h_ppa = pr.a, &h_ppb = pr.b, &h_sign = pr.sign;
+  const auto &h_coff = pr.c_off, &h_ma = pr.m, &h_ka = pr.k, &h_nb = pr.n;
 
   // Result blocks (ascending block index) and offsets.
   C.nblk = ncb;

@@ -64,10 +64,22 @@ class DevBuf {
   ~DevBuf() { release(); }
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
-  DevBuf(DevBuf&& o) noexcept : p_(o.p_), n_(o.n_) { o.p_ = nullptr; o.n_ = 0; }
+  DevBuf(DevBuf&& o) noexcept : p_(o.p_), n_(o.n_), own_(o.own_) { o.p_ = nullptr; o.n_ = 0; o.own_ = true; }
   DevBuf& operator=(DevBuf&& o) noexcept {
-    if (this != &o) { release(); p_ = o.p_; n_ = o.n_; o.p_ = nullptr; o.n_ = 0; }
+    if (this != &o) {
+      release();
+      p_ = o.p_; n_ = o.n_; own_ = o.own_;
+      o.p_ = nullptr; o.n_ = 0; o.own_ = true;
+    }
     return *this;
+  }
+  // A range of another buffer, which has to outlive this one.
+  static DevBuf part(const DevBuf& whole, size_t offset, size_t bytes) {
+    DevBuf b;
+    b.p_ = static_cast<char*>(whole.p_) + offset;
+    b.n_ = bytes;
+    b.own_ = false;
+    return b;
   }
   void alloc(size_t bytes) {
     release();
@@ -75,9 +87,10 @@ class DevBuf {
     n_ = bytes;
   }
   void release() {
-    if (p_) cudaFree(p_);
+    if (p_ && own_) cudaFree(p_);
     p_ = nullptr;
     n_ = 0;
+    own_ = true;
   }
   template <typename T> T* as() const { return static_cast<T*>(p_); }
   void* get() const { return p_; }
@@ -86,6 +99,7 @@ class DevBuf {
  private:
   void* p_ = nullptr;
   size_t n_ = 0;
+  bool own_ = true;
 };
 
 // Streaming multiprocessors of the current device (grid sizing for kernels launched without
@@ -154,4 +168,14 @@ struct qltg_ctx {
   int device = 0;
   int num_sms = 0;
   int cc_major = 0, cc_minor = 0;
+  // Work of plan creation (uploads, device pairing): a stream of its own, so that planning does
+  // not wait for what the caller's streams have queued. Shared by the context's threads; every
+  // user waits for it before returning.
+  cudaStream_t plan_stream = nullptr;
+  // Held for the context's life: small allocations come from 2 MB pieces that the driver maps and
+  // unmaps, and while one is in use a small cudaMalloc + cudaFree takes 6 us instead of 62.
+  qltg::DevBuf small_piece;
+  ~qltg_ctx() {
+    if (plan_stream) cudaStreamDestroy(plan_stream);
+  }
 };

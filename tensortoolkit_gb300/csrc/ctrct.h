@@ -77,10 +77,18 @@ struct GemmTileRun {
   int32_t cblk, begin;
   int32_t tm0, tn0, tn_count;
 };
-struct GemmRowChunk {          // skinny output blocks: 256 consecutive rows of one block
-  int32_t cblk;
-  int32_t chunk;
+// Skinny output blocks (n, k <= 8): a piece of a block's m x n outputs (skinny_outputs of them from
+// o0) and the block's entries [e0, e1), its tasks' k values laid end to end: the A column (element
+// (row) at a_off + row a_rs) and the B row (n values at b_off) that each multiplies.
+struct SkinnyItem {
+  int32_t cblk, o0, e0, e1;
 };
+struct SkinnyEntry {
+  int64_t a_off, b_off;        // | kFromSrc
+  int32_t a_rs, sign;
+  int64_t pad;
+};
+static_assert(sizeof(SkinnyItem) == 16 && sizeof(SkinnyEntry) == 32, "records of one or two 16-byte loads");
 
 // Row-scale fields of a later split-mode contraction's A operand, folded by the skinny kernel
 // that writes that operand (the matvec's second MPO step writing the last step's A): per
@@ -97,11 +105,12 @@ struct GemmSchedule {
   std::vector<GemmTileRun> run;         // FP64 warp tiles, longest first
   int64_t ntiles = 0;                   // tiles of all runs
   bool share_tiles = false;             // a CTA's warps share each tile (few or very long tiles)
-  std::vector<GemmRowChunk> skinny;     // row chunks of skinny blocks (n, k <= 8)
+  std::vector<SkinnyItem> skinny;       // pieces of skinny blocks (n, k <= 8)
+  std::vector<SkinnyEntry> skinny_entry;
+  int skinny_outputs = 128;             // outputs of an item (the last of a block may have fewer)
   DevBuf lists;                          // holds the device copies below (parts of it)
-  DevBuf d_cblk, d_task, d_run, d_skinny, d_counter;
+  DevBuf d_cblk, d_task, d_run, d_skinny, d_entry, d_counter;
   int bm = 32;                          // rows of the FP64 tiles of a CTA's four warps
-  int skinny_maxn = 8;                  // largest n of the skinny blocks (kernel variant)
 };
 
 // Split-precision schedule (gemm_split.cu): operand blocks to slice and pack, per-task
@@ -236,10 +245,9 @@ void exec_contraction(CtrctPlan& p, const void* a, const void* b, void* c, int m
 // grouped GEMM launchers (gemm_f64.cu)
 constexpr int kF64TileCols = 16;   // columns of an FP64 warp tile
 bool skinny_cblk(const GemmSchedule& g, int32_t q);
-int skinny_rows_per_item();
 // Grid of the skinny kernel: one full wave of resident CTAs (the first call queries the
 // occupancy; call it once outside any stream capture).
-int skinny_grid(int items, bool cplx, int maxn, int num_sms);
+int skinny_grid(int items, bool cplx, int num_sms);
 // Operand buffers of one execution: scratch (transposed blocks) and source (the operands as
 // passed in, for blocks flagged kFromSrc).
 struct Operands {

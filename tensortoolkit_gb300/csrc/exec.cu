@@ -64,18 +64,41 @@ void set_f64_tile(CtrctPlan& p, int bm, cudaStream_t s) {
   QLTG_CUDA(cudaStreamSynchronize(s));
 }
 
+// Entries and pieces of the skinny blocks (the tasks' operand offsets are final). An item is one
+// pass of a warp, 128 outputs; where there are very many passes and blocks are large enough for it
+// to add under a quarter of empty ones, an item stands for four passes, to keep the list short.
+static void skinny_list(GemmSchedule& g, int num_sms) {
+  int64_t passes = 0, items = 0;
+  for (int32_t q = 0; q < (int32_t)g.cblk.size(); ++q) {
+    if (!skinny_cblk(g, q)) continue;
+    const int64_t outputs = (int64_t)g.cblk[q].m * g.cblk[q].n;
+    QLTG_CHECK(outputs < ((int64_t)1 << 31) - 512, QLTG_ERR_UNSUPPORTED, "output block too large");
+    passes += (outputs + 127) / 128;
+    items += (outputs + 511) / 512;
+  }
+  g.skinny_outputs = passes > (int64_t)num_sms * 32 * 4 && 16 * items <= 5 * passes ? 512 : 128;
+  QLTG_CHECK(4 * items < ((int64_t)1 << 31) && passes < ((int64_t)1 << 31), QLTG_ERR_UNSUPPORTED, "too many rows of small blocks");
+  for (int32_t q = 0; q < (int32_t)g.cblk.size(); ++q) {
+    if (!skinny_cblk(g, q)) continue;
+    const GemmCBlk& cb = g.cblk[q];
+    const size_t e0 = g.skinny_entry.size();
+    for (int32_t t = cb.t0; t < cb.t1; ++t) {
+      const GemmTask& tk = g.task[t];
+      for (int32_t kk = 0; kk < tk.k; ++kk)
+        g.skinny_entry.push_back(SkinnyEntry{tk.a_off + (int64_t)kk * tk.a_cs, tk.b_off + (int64_t)kk * cb.n, tk.a_rs, tk.sign, 0});
+    }
+    QLTG_CHECK(g.skinny_entry.size() < ((size_t)1 << 31), QLTG_ERR_UNSUPPORTED, "too many small tasks");
+    for (int64_t o = 0; o < (int64_t)cb.m * cb.n; o += g.skinny_outputs)
+      g.skinny.push_back(SkinnyItem{q, (int32_t)o, (int32_t)e0, (int32_t)g.skinny_entry.size()});
+  }
+}
+
 void finalize_plan(CtrctPlan& p, cudaStream_t s) {
   GemmSchedule& g = p.sched;
   g.skinny.clear();
-  g.skinny_maxn = 1;
-  const int rows_per_item = skinny_rows_per_item();
-  for (int32_t q = 0; q < (int32_t)g.cblk.size(); ++q) {
-    const GemmCBlk& cb = g.cblk[q];
-    if (skinny_cblk(g, q)) {
-      g.skinny_maxn = std::max(g.skinny_maxn, (int)cb.n);
-      for (int32_t c = 0; c * (int64_t)rows_per_item < cb.m; ++c) g.skinny.push_back(GemmRowChunk{q, c});
-    }
-  }
+  g.skinny_entry.clear();
+  bool any_skinny = false;
+  for (int32_t q = 0; q < (int32_t)g.cblk.size(); ++q) any_skinny |= skinny_cblk(g, q);
   f64_tile_list(g, p.ctx->num_sms);
   // Operand transposes. A task reads its operand block from the transposed scratch unless
   // (a) the permutation leaves the block's layout unchanged, or (b) it is a skinny task and
@@ -83,7 +106,7 @@ void finalize_plan(CtrctPlan& p, cudaStream_t s) {
   // tasks read the operand itself (offset flag kFromSrc) and blocks nobody reads from the
   // scratch get no transpose work.
   const size_t eb = p.a.elem_bytes();
-  const bool any_work = g.ntiles || !g.skinny.empty();
+  const bool any_work = g.ntiles || any_skinny;
   std::vector<uint8_t> skinny_task(g.task.size(), 0);
   for (int32_t q = 0; q < (int32_t)g.cblk.size(); ++q)
     if (skinny_cblk(g, q))
@@ -154,14 +177,16 @@ void finalize_plan(CtrctPlan& p, cudaStream_t s) {
       if (p.b_tl.identity[block_of(p.b, tk.b_off)]) tk.b_off |= kFromSrc;
     if (p.b_tl.ntiles) p.b_t.alloc(p.b.size * eb);
   }
-  if (!g.skinny.empty()) (void)skinny_grid((int)g.skinny.size(), p.a.dtype == QLTG_C128, g.skinny_maxn, p.ctx->num_sms);
+  if (any_skinny) skinny_list(g, p.ctx->num_sms);
+  if (any_skinny) (void)skinny_grid((int)g.skinny.size(), p.a.dtype == QLTG_C128, p.ctx->num_sms);
   // the schedule's lists in one buffer, with one copy
   {
     const struct { const void* src; size_t bytes; DevBuf* part; } lists[] = {
         {g.cblk.data(), g.cblk.size() * sizeof(GemmCBlk), &g.d_cblk},
         {g.task.data(), g.task.size() * sizeof(GemmTask), &g.d_task},
         {g.run.data(), g.run.size() * sizeof(GemmTileRun), &g.d_run},
-        {g.skinny.data(), g.skinny.size() * sizeof(GemmRowChunk), &g.d_skinny},
+        {g.skinny.data(), g.skinny.size() * sizeof(SkinnyItem), &g.d_skinny},
+        {g.skinny_entry.data(), g.skinny_entry.size() * sizeof(SkinnyEntry), &g.d_entry},
         {nullptr, sizeof(int), &g.d_counter}};
     auto room = [](size_t n) { return (n + 255) / 256 * 256; };
     size_t total = 0;

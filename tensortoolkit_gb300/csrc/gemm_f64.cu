@@ -13,8 +13,7 @@
 //                    DFMA (about 1.05 TFLOP/s each, measured) but pads every block to 8 x 8 x 4
 //                    fragments, so predicated DFMA is the faster FP64 kernel;
 //  * k_gemm_skinny - output blocks with n <= 8 and k <= 8 (the MPO steps of the two-site
-//                    matvec: m up to 3e4, k, n <= 3): one thread per output row, operand B
-//                    in registers, memory-streaming.
+//                    matvec: m up to 3e4, k, n <= 3): one output per lane, memory-streaming.
 #include <algorithm>
 
 #include "ctrct.h"
@@ -194,14 +193,22 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 8 ? (TM == 1 ? 4 : 3) : 2) k_
   }
 }
 
-// Skinny output blocks (n <= 8, every task k <= 8): the rows' n outputs in registers,
-// instantiated per n so no FP64 slot is spent on absent columns. A work item is 256 rows of
-// one block; each of the 128 threads takes rows r and r + 128, both in one pass over the
-// tasks when n <= 4 (real): the task records and B values are loaded once for two rows and
-// two independent FMA chains hide each other's load latency.
-constexpr int kSkinnyRows = 256;
+// Skinny output blocks (n <= 8, every task k <= 8). An FP64 instruction costs the same whatever
+// lanes are active, so a block's m x n outputs are taken as one flat range, one per lane and up to
+// four ranges of 32 at once: every lane has an output whatever m and n are, and the stores are
+// contiguous. Operand reads are cheap beside that (lanes of one row share an address). The block's
+// entries (its tasks' k values end to end) are worked off kSkinnyDepth at a time: their records,
+// then all their A and B values, then the multiply-adds, so a pass waits about twice for memory
+// and not twice per task; the next pass's record is read ahead. Bound by the FP64 pipe where a
+// launch has enough passes, else by those waits.
+// Measured against one thread per row (256 rows per CTA, n columns in registers): MPO part of the
+// D = 4000 matvec 126 -> 118 us (114 us of multiply-adds at the pipe's rate), the two MPO steps of
+// the D = 3000 complex Hubbard matvec 245 -> 145 us, its blocks of a few rows 171 -> 64 us. Depth 1
+// / 2 / 3 / 4: 401 / 390 / 393 / 399 us per D = 4000 matvec.
 constexpr int kSkinnyThreads = 128;
 constexpr int kSkinnyMax = 8;
+constexpr int kSkinnyPass = 128;   // outputs of one pass
+constexpr int kSkinnyDepth = 2;
 
 // Scale field of an output value as the split path defines it (0 for zero, else
 // max(1, biased exponent)); complex outputs are never folded.
@@ -211,97 +218,6 @@ __device__ __forceinline__ int out_field(double v) {
 }
 __device__ __forceinline__ int out_field(double2 v) { return max(out_field(v.x), out_field(v.y)); }
 
-template <typename T, int NN>
-__device__ __forceinline__ void skinny_row(const GemmCBlk& cb, const GemmTask* __restrict__ task, int row,
-                                           const T* __restrict__ A, const T* __restrict__ As, const T* __restrict__ B,
-                                           const T* __restrict__ Bs, T* __restrict__ C, bool want, int& f) {
-  T acc[NN];
-#pragma unroll
-  for (int j = 0; j < NN; ++j) acc[j] = zero_of(T());
-  for (int t = cb.t0; t < cb.t1; ++t) {
-    const GemmTask tk = task[t];
-    const int k = tk.k;
-    const T* a = operand_block(A, As, tk.a_off) + (int64_t)row * tk.a_rs;
-    const T* b = operand_block(B, Bs, tk.b_off);
-    const unsigned long long sg = sign_mask(tk.sign);
-    for (int kk = 0; kk < k; ++kk) {
-      const T av = flip(__ldg(a + (int64_t)kk * tk.a_cs), sg);
-#pragma unroll
-      for (int j = 0; j < NN; ++j) fma_acc(acc[j], av, __ldg(b + kk * NN + j));
-    }
-  }
-  T* out = C + cb.c_off + (int64_t)row * NN;
-#pragma unroll
-  for (int j = 0; j < NN; ++j) out[j] = acc[j];
-  if (want) {
-    f = 0;
-#pragma unroll
-    for (int j = 0; j < NN; ++j) f = max(f, out_field(acc[j]));
-  }
-}
-
-// Rows row0 and row0 + kSkinnyThreads (both inside the block) in one pass.
-template <typename T, int NN>
-__device__ __forceinline__ void skinny_row_pair(const GemmCBlk& cb, const GemmTask* __restrict__ task, int row0,
-                                                const T* __restrict__ A, const T* __restrict__ As,
-                                                const T* __restrict__ B, const T* __restrict__ Bs,
-                                                T* __restrict__ C, bool want, int& f0, int& f1) {
-  T acc0[NN], acc1[NN];
-#pragma unroll
-  for (int j = 0; j < NN; ++j) acc0[j] = acc1[j] = zero_of(T());
-  for (int t = cb.t0; t < cb.t1; ++t) {
-    const GemmTask tk = task[t];
-    const int k = tk.k;
-    const T* a0 = operand_block(A, As, tk.a_off) + (int64_t)row0 * tk.a_rs;
-    const T* a1 = a0 + (int64_t)kSkinnyThreads * tk.a_rs;
-    const T* b = operand_block(B, Bs, tk.b_off);
-    const unsigned long long sg = sign_mask(tk.sign);
-    for (int kk = 0; kk < k; ++kk) {
-      const T x0 = flip(__ldg(a0 + (int64_t)kk * tk.a_cs), sg);
-      const T x1 = flip(__ldg(a1 + (int64_t)kk * tk.a_cs), sg);
-#pragma unroll
-      for (int j = 0; j < NN; ++j) {
-        const T bj = __ldg(b + kk * NN + j);
-        fma_acc(acc0[j], x0, bj);
-        fma_acc(acc1[j], x1, bj);
-      }
-    }
-  }
-  T* out0 = C + cb.c_off + (int64_t)row0 * NN;
-  T* out1 = out0 + (int64_t)kSkinnyThreads * NN;
-#pragma unroll
-  for (int j = 0; j < NN; ++j) {
-    out0[j] = acc0[j];
-    out1[j] = acc1[j];
-  }
-  if (want) {
-    f0 = f1 = 0;
-#pragma unroll
-    for (int j = 0; j < NN; ++j) {
-      f0 = max(f0, out_field(acc0[j]));
-      f1 = max(f1, out_field(acc1[j]));
-    }
-  }
-}
-
-// Row row0 of an item and, if inside the block, row0 + kSkinnyThreads.
-// f0, f1: the rows' output fields when `want` (f1 stays -1 when row1 is outside the block).
-template <typename T, int NN>
-__device__ __forceinline__ void skinny_rows(const GemmCBlk& cb, const GemmTask* __restrict__ task, int row0,
-                                            const T* __restrict__ A, const T* __restrict__ As, const T* __restrict__ B,
-                                            const T* __restrict__ Bs, T* __restrict__ C, bool want, int& f0,
-                                            int& f1) {
-  const int row1 = row0 + kSkinnyThreads;
-  if constexpr (sizeof(T) == 8 && NN <= 4) {
-    if (row1 < cb.m) {
-      skinny_row_pair<T, NN>(cb, task, row0, A, As, B, Bs, C, want, f0, f1);
-      return;
-    }
-  }
-  skinny_row<T, NN>(cb, task, row0, A, As, B, Bs, C, want, f0);
-  if (row1 < cb.m) skinny_row<T, NN>(cb, task, row1, A, As, B, Bs, C, want, f1);
-}
-
 // atomicMax of v into fields[key] once per group of lanes with the same key.
 __device__ __forceinline__ void fold_field(unsigned mask, int key, int v, int32_t* __restrict__ fields) {
   const unsigned m = __match_any_sync(mask, key);
@@ -309,56 +225,83 @@ __device__ __forceinline__ void fold_field(unsigned mask, int key, int v, int32_
   if (key >= 0 && x > 0 && (int)(threadIdx.x & 31) == __ffs(m) - 1) atomicMax(fields + key, x);
 }
 
-// Resident CTAs per SM the kernel is compiled for: 8 for real operands (64 registers, no
-// spills at two rows per thread); complex ones need their registers, the more the wider the
-// blocks (the kernel is instantiated for the plan's largest n: MAXN = 2, 4 or 8).
-template <typename T, int MAXN> struct SkinnyMinBlocks { static constexpr int value = MAXN <= 2 ? 6 : MAXN <= 4 ? 4 : 2; };
-template <int MAXN> struct SkinnyMinBlocks<double, MAXN> { static constexpr int value = 8; };
-
-template <typename T, int MAXN>
-__global__ void __launch_bounds__(kSkinnyThreads, SkinnyMinBlocks<T, MAXN>::value) k_gemm_skinny(
-    const GemmCBlk* __restrict__ cblk, const GemmTask* __restrict__ task, const GemmRowChunk* __restrict__ items,
-    int nitems, const T* __restrict__ A, const T* __restrict__ As, const T* __restrict__ B, const T* __restrict__ Bs,
-    T* __restrict__ C, const SkinnyFuse* __restrict__ fuse, int32_t* __restrict__ fields) {
-  for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-    const GemmRowChunk item = items[it];
-    const GemmCBlk cb = cblk[item.cblk];
-    const int row = item.chunk * kSkinnyRows + threadIdx.x;
-    if (row >= cb.m) continue;
-    const SkinnyFuse fz = fuse ? fuse[item.cblk] : SkinnyFuse{-1, 1};
-    const bool want = fz.exp_base >= 0;   // uniform over the item
-    int f0 = 0, f1 = -1;
-    if (MAXN <= 2) {
-      if (cb.n == 1) skinny_rows<T, 1>(cb, task, row, A, As, B, Bs, C, want, f0, f1);
-      else skinny_rows<T, 2>(cb, task, row, A, As, B, Bs, C, want, f0, f1);
-    } else if (MAXN <= 4) {
-      switch (cb.n) {
-        case 1: skinny_rows<T, 1>(cb, task, row, A, As, B, Bs, C, want, f0, f1); break;
-        case 2: skinny_rows<T, 2>(cb, task, row, A, As, B, Bs, C, want, f0, f1); break;
-        case 3: skinny_rows<T, 3>(cb, task, row, A, As, B, Bs, C, want, f0, f1); break;
-        default: skinny_rows<T, 4>(cb, task, row, A, As, B, Bs, C, want, f0, f1); break;
-      }
-    } else {
-      switch (cb.n) {
-        case 1: skinny_rows<T, 1>(cb, task, row, A, As, B, Bs, C, want, f0, f1); break;
-        case 2: skinny_rows<T, 2>(cb, task, row, A, As, B, Bs, C, want, f0, f1); break;
-        case 3: skinny_rows<T, 3>(cb, task, row, A, As, B, Bs, C, want, f0, f1); break;
-        case 4: skinny_rows<T, 4>(cb, task, row, A, As, B, Bs, C, want, f0, f1); break;
-        case 5: skinny_rows<T, 5>(cb, task, row, A, As, B, Bs, C, want, f0, f1); break;
-        case 6: skinny_rows<T, 6>(cb, task, row, A, As, B, Bs, C, want, f0, f1); break;
-        case 7: skinny_rows<T, 7>(cb, task, row, A, As, B, Bs, C, want, f0, f1); break;
-        default: skinny_rows<T, 8>(cb, task, row, A, As, B, Bs, C, want, f0, f1); break;
+// Outputs o + lane + 32 u (u < U, clamped into the block) of one block, from all its entries.
+template <typename T, int U>
+__device__ __forceinline__ void skinny_pass(const GemmCBlk& cb, const SkinnyItem& item, int o, int lane,
+                                            const SkinnyEntry* __restrict__ entry, const T* __restrict__ A,
+                                            const T* __restrict__ As, const T* __restrict__ B, const T* __restrict__ Bs,
+                                            T* __restrict__ C, const SkinnyFuse& fz, int32_t* __restrict__ fields) {
+  const int total = cb.m * cb.n;
+  int row[U], col[U];
+  T acc[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int x = min(o + 32 * u + lane, total - 1);
+    row[u] = x / cb.n;
+    col[u] = x - row[u] * cb.n;
+    acc[u] = zero_of(T());
+  }
+  int e = item.e0;
+  for (; e + kSkinnyDepth <= item.e1; e += kSkinnyDepth) {
+    T av[kSkinnyDepth][U], bv[kSkinnyDepth][U];
+#pragma unroll
+    for (int t = 0; t < kSkinnyDepth; ++t) {
+      const SkinnyEntry x = entry[e + t];
+      const T* a = operand_block(A, As, x.a_off);
+      const T* b = operand_block(B, Bs, x.b_off);
+      const unsigned long long sg = sign_mask(x.sign);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        av[t][u] = flip(__ldg(a + (int64_t)row[u] * x.a_rs), sg);
+        bv[t][u] = __ldg(b + col[u]);
       }
     }
-    if (want) {
-      // a row's n outputs lie in one row of the later operand (k3 is a multiple of n)
-      const unsigned mask = __activemask();
-      fold_field(mask, fz.exp_base + row * cb.n / fz.k3, f0, fields);
-      fold_field(mask, f1 >= 0 ? fz.exp_base + (row + kSkinnyThreads) * cb.n / fz.k3 : -1, f1, fields);
-    }
+#pragma unroll
+    for (int t = 0; t < kSkinnyDepth; ++t)
+#pragma unroll
+      for (int u = 0; u < U; ++u) fma_acc(acc[u], av[t][u], bv[t][u]);
+  }
+#pragma unroll 1
+  for (; e < item.e1; ++e) {   // a loop: predicated-off multiply-adds would cost as much as executed ones
+    const SkinnyEntry x = entry[e];
+    const T* a = operand_block(A, As, x.a_off);
+    const T* b = operand_block(B, Bs, x.b_off);
+    const unsigned long long sg = sign_mask(x.sign);
+#pragma unroll
+    for (int u = 0; u < U; ++u) fma_acc(acc[u], flip(__ldg(a + (int64_t)row[u] * x.a_rs), sg), __ldg(b + col[u]));
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int x = o + 32 * u + lane;
+    if (x < total) C[cb.c_off + x] = acc[u];
+    // the outputs' order is that of the later operand's rows of k3 values
+    if (fz.exp_base >= 0) fold_field(0xffffffffu, x < total ? fz.exp_base + x / fz.k3 : -1, out_field(acc[u]), fields);
   }
 }
 
+template <typename T>
+__global__ void __launch_bounds__(kSkinnyThreads, sizeof(T) == 8 ? 7 : 5) k_gemm_skinny(
+    const GemmCBlk* __restrict__ cblk, const SkinnyEntry* __restrict__ entry, const SkinnyItem* __restrict__ items,
+    int npasses, int shift, const T* __restrict__ A, const T* __restrict__ As, const T* __restrict__ B,
+    const T* __restrict__ Bs, T* __restrict__ C, const SkinnyFuse* __restrict__ fuse, int32_t* __restrict__ fields) {
+  const int lane = threadIdx.x & 31, step = gridDim.x * (kSkinnyThreads / 32);
+  int it = blockIdx.x * (kSkinnyThreads / 32) + (threadIdx.x >> 5);
+  if (it >= npasses) return;
+  SkinnyItem next = items[it >> shift];
+  for (; it < npasses; it += step) {
+    const SkinnyItem item = next;
+    const int o = item.o0 + (it & ((1 << shift) - 1)) * kSkinnyPass;
+    if (it + step < npasses) next = items[(it + step) >> shift];
+    const GemmCBlk cb = cblk[item.cblk];
+    const int left = cb.m * cb.n - o;
+    if (left <= 0) continue;
+    const SkinnyFuse fz = fuse ? fuse[item.cblk] : SkinnyFuse{-1, 1};
+    if (left > 96) skinny_pass<T, 4>(cb, item, o, lane, entry, A, As, B, Bs, C, fz, fields);
+    else if (left > 64) skinny_pass<T, 3>(cb, item, o, lane, entry, A, As, B, Bs, C, fz, fields);
+    else if (left > 32) skinny_pass<T, 2>(cb, item, o, lane, entry, A, As, B, Bs, C, fz, fields);
+    else skinny_pass<T, 1>(cb, item, o, lane, entry, A, As, B, Bs, C, fz, fields);
+  }
+}
 
 }  // namespace
 
@@ -370,16 +313,14 @@ bool skinny_cblk(const GemmSchedule& g, int32_t q) {
   return true;
 }
 
-int skinny_rows_per_item() { return kSkinnyRows; }
-
-template <typename T, int MAXN>
-void launch_skinny_t(const GemmSchedule& g, const Operands& op, void* c, int grid, cudaStream_t s,
-                     const SkinnyFuse* fuse, int32_t* fields) {
-  k_gemm_skinny<T, MAXN><<<grid, kSkinnyThreads, 0, s>>>(g.d_cblk.as<GemmCBlk>(), g.d_task.as<GemmTask>(),
-                                                   g.d_skinny.as<GemmRowChunk>(), (int)g.skinny.size(),
-                                                   static_cast<const T*>(op.a), static_cast<const T*>(op.a_src),
-                                                   static_cast<const T*>(op.b), static_cast<const T*>(op.b_src),
-                                                   static_cast<T*>(c), fuse, fields);
+template <typename T>
+void launch_skinny(const GemmSchedule& g, const Operands& op, void* c, int grid, cudaStream_t s, const SkinnyFuse* fuse,
+                   int32_t* fields) {
+  const int shift = g.skinny_outputs == 4 * kSkinnyPass ? 2 : 0;
+  k_gemm_skinny<T><<<grid, kSkinnyThreads, 0, s>>>(
+      g.d_cblk.as<GemmCBlk>(), g.d_entry.as<SkinnyEntry>(), g.d_skinny.as<SkinnyItem>(), (int)g.skinny.size() << shift,
+      shift, static_cast<const T*>(op.a), static_cast<const T*>(op.a_src), static_cast<const T*>(op.b),
+      static_cast<const T*>(op.b_src), static_cast<T*>(c), fuse, fields);
 }
 
 template <typename T, int TM, bool SHARE>
@@ -404,42 +345,29 @@ void launch_f64(const GemmSchedule& g, const Operands& op, void* c, int num_sms,
 }
 
 // CTAs of one full wave: the grid-stride loop then has no partial second wave.
-template <typename T, int MAXN>
+template <typename T>
 int skinny_wave(int num_sms) {
   static int per_sm = [] {
     int n = 0;
-    QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_gemm_skinny<T, MAXN>, kSkinnyThreads, 0));
+    QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_gemm_skinny<T>, kSkinnyThreads, 0));
     return std::max(1, n);
   }();
   return std::max(1, num_sms) * per_sm;
 }
 
-// the kernel variant of a plan: real operands always use MAXN = 8 (64 registers either way);
-// complex ones the narrowest that covers the plan's blocks
-int skinny_variant(bool cplx, int maxn) { return !cplx ? 8 : maxn <= 2 ? 2 : maxn <= 4 ? 4 : 8; }
-
-int skinny_grid(int items, bool cplx, int maxn, int num_sms) {
-  int wave = 0;
-  switch (skinny_variant(cplx, maxn)) {
-    case 2: wave = skinny_wave<double2, 2>(num_sms); break;
-    case 4: wave = skinny_wave<double2, 4>(num_sms); break;
-    default: wave = cplx ? skinny_wave<double2, 8>(num_sms) : skinny_wave<double, 8>(num_sms); break;
-  }
-  return std::max(1, std::min(items, wave));
+int skinny_grid(int items, bool cplx, int num_sms) {
+  const int wave = cplx ? skinny_wave<double2>(num_sms) : skinny_wave<double>(num_sms);
+  const int per_cta = kSkinnyThreads / 32;
+  return std::max(1, std::min((items + per_cta - 1) / per_cta, wave));
 }
 
 void launch_gemm_f64_skinny(const GemmSchedule& g, const Operands& op, void* c, bool cplx, int num_sms,
                             cudaStream_t s, const SkinnyFuse* fuse, int32_t* fields) {
   const int ns = (int)g.skinny.size();
   if (!ns) return;
-  const int grid = skinny_grid(ns, cplx, g.skinny_maxn, num_sms);
-  switch (skinny_variant(cplx, g.skinny_maxn)) {
-    case 2: launch_skinny_t<double2, 2>(g, op, c, grid, s, fuse, fields); break;
-    case 4: launch_skinny_t<double2, 4>(g, op, c, grid, s, fuse, fields); break;
-    default:
-      if (cplx) launch_skinny_t<double2, 8>(g, op, c, grid, s, fuse, fields);
-      else launch_skinny_t<double, 8>(g, op, c, grid, s, fuse, fields);
-  }
+  const int grid = skinny_grid(ns, cplx, num_sms);
+  if (cplx) launch_skinny<double2>(g, op, c, grid, s, fuse, fields);
+  else launch_skinny<double>(g, op, c, grid, s, fuse, fields);
   QLTG_CUDA(cudaGetLastError());
 }
 

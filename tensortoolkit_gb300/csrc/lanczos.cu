@@ -20,6 +20,7 @@
 // on first use.
 #include <cmath>
 #include <memory>
+#include <type_traits>
 
 #include "matvec.h"
 
@@ -28,24 +29,12 @@ using namespace qltg;
 namespace {
 
 constexpr int kVecThreads = 256;
+constexpr int kVecWarps = kVecThreads / 32;
 // fixed grid, deliberately independent of the device's SM count: the partial-sum order, and
-// so every α and β, is the same on every run and every GPU (608 CTAs = four per SM on a
-// 152-SM GB300)
-constexpr int kVecBlocks = 608;
-
-__device__ __forceinline__ double block_sum(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (warp == 0) {
-    t = lane < (int)(blockDim.x >> 5) ? red[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  }
-  __syncthreads();
-  return t;   // valid in thread 0
-}
+// so every α and β, is the same on every run and every GPU (304 CTAs = two per SM on a
+// 152-SM GB300; every CTA's sums cost it about 150 FP64 instructions, so not more)
+constexpr int kVecBlocks = 304;
+constexpr int kGroup = 8;   // sums formed at once: 8 real or 4 complex dots
 
 // Scalar algebra of the two vector kinds: real FP64 (double) and complex128 (double2).
 struct RealOps {
@@ -68,102 +57,178 @@ struct ComplexOps {
   }
 };
 
-// N sums at once: one warp shuffle tree each, one shared-memory round for all (valid in
-// thread 0). The per-value order is fixed, as in block_sum.
+// The sums of v[0 .. N) (N a power of two) over the warp's lanes: lane l gets the one of index
+// sum_index<N>(l). Halves are exchanged while they are added, so N sums take N + 5 - log2 N - 1
+// additions and not 5 N (an FP64 addition costs a warp 80 cycles here). Fixed order.
 template <int N>
-__device__ __forceinline__ void block_sum_n(double (&v)[N], double* red) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+__device__ __forceinline__ double warp_sums(double (&v)[N], int lane) {
+  int o = 16;
 #pragma unroll
-  for (int i = 0; i < N; ++i) {
-    for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
-    if (lane == 0) red[i * (kVecThreads / 32) + warp] = v[i];
-  }
-  __syncthreads();
-  if (warp == 0) {
+  for (int w = N / 2; w >= 1; w /= 2, o /= 2) {
+    const bool up = lane & o;
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-      double t = lane < nw ? red[i * (kVecThreads / 32) + lane] : 0.0;
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      v[i] = t;
+    for (int k = 0; k < w; ++k) {
+      const double send = up ? v[k] : v[k + w], keep = up ? v[k + w] : v[k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
+  }
+  for (; o > 0; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+template <int N>
+__device__ __forceinline__ int sum_index(int lane) {
+  int i = 0, o = 16;
+#pragma unroll
+  for (int w = N / 2; w >= 1; w /= 2, o /= 2) i += lane & o ? w : 0;
+  return i;
+}
+
+__host__ __device__ constexpr int pow2_up(int n) { return n <= 1 ? 1 : n <= 2 ? 2 : n <= 4 ? 4 : 8; }
+
+// part[value * gridDim.x + CTA] = this CTA's share of conj(V_i) w for the G vectors from V (its
+// elements [e0, e1), a thread's own ones). One instantiation per G: a predicated-off multiply-add
+// would cost as much as an executed one.
+template <class Ops, int G>
+__device__ __forceinline__ void dot_group(const typename Ops::T* __restrict__ V, int64_t ld,
+                                          const typename Ops::T* __restrict__ w, int64_t e0, int64_t e1,
+                                          double (*red)[kGroup], double* __restrict__ part) {
+  constexpr int N = G * Ops::kParts, P = pow2_up(N);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double acc[P] = {};
+#pragma unroll 2
+  for (int64_t e = e0 + threadIdx.x; e < e1; e += kVecThreads) {
+    const typename Ops::T x = w[e];
+    typename Ops::T v[G];
+#pragma unroll
+    for (int u = 0; u < G; ++u) v[u] = __ldg(V + (int64_t)u * ld + e);
+#pragma unroll
+    for (int u = 0; u < G; ++u) Ops::dot_acc(v[u], x, acc + u * Ops::kParts);
+  }
+  const double t = warp_sums<P>(acc, lane);
+  if ((lane & (32 / P - 1)) == 0) red[warp][sum_index<P>(lane)] = t;
+  __syncthreads();
+  if (threadIdx.x < N) {
+    double s = red[0][threadIdx.x];
+#pragma unroll
+    for (int q = 1; q < kVecWarps; ++q) s += red[q][threadIdx.x];
+    part[(int64_t)threadIdx.x * gridDim.x + blockIdx.x] = s;
   }
   __syncthreads();
 }
 
-// part[(i * gridDim.x + b) * kParts + r] = part r of the sum over CTA b's chunk of conj(V_i[e]) w[e].
-// Four vectors per pass over the chunk: w is loaded once for them, and the four load streams
-// keep more reads in flight than one vector at a time.
-template <class Ops>
-__global__ void __launch_bounds__(kVecThreads) k_multi_dot(const typename Ops::T* __restrict__ V, int nv, int64_t ld,
-                                                           const typename Ops::T* __restrict__ w, int64_t n,
-                                                           double* __restrict__ part) {
-  constexpr int kG = 4, kN = kG * Ops::kParts;
-  __shared__ double red[kN * (kVecThreads / 32)];
-  const int64_t per = (n + gridDim.x - 1) / gridDim.x;
-  const int64_t e0 = (int64_t)blockIdx.x * per, e1 = min(n, e0 + per);
-  for (int i0 = 0; i0 < nv; i0 += kG) {
-    const int g = min(kG, nv - i0);
-    double acc[kG][Ops::kParts] = {};
-    for (int64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-      const typename Ops::T x = __ldg(w + e);
+// x - sum over G vectors of c_i V_i, for this thread's elements.
+template <class Ops, int G>
+__device__ __forceinline__ void subtract_group(const typename Ops::T* __restrict__ V, int64_t ld, const double* c,
+                                               typename Ops::T* __restrict__ w, int64_t e0, int64_t e1) {
+  double k[G * Ops::kParts];
 #pragma unroll
-      for (int u = 0; u < kG; ++u)
-        if (u < g) Ops::dot_acc(__ldg(V + (int64_t)(i0 + u) * ld + e), x, acc[u]);
-    }
-    double flat[kN];
+  for (int u = 0; u < G * Ops::kParts; ++u) k[u] = c[u];
+#pragma unroll 2
+  for (int64_t e = e0 + threadIdx.x; e < e1; e += kVecThreads) {
+    typename Ops::T x = w[e], v[G];
 #pragma unroll
-    for (int u = 0; u < kG; ++u)
+    for (int u = 0; u < G; ++u) v[u] = __ldg(V + (int64_t)u * ld + e);
 #pragma unroll
-      for (int r = 0; r < Ops::kParts; ++r) flat[u * Ops::kParts + r] = acc[u][r];
-    block_sum_n<kN>(flat, red);
-    if (threadIdx.x == 0)
-      for (int u = 0; u < g; ++u)
-        for (int r = 0; r < Ops::kParts; ++r)
-          part[((int64_t)(i0 + u) * gridDim.x + blockIdx.x) * Ops::kParts + r] = flat[u * Ops::kParts + r];
-  }
-}
-
-// c[i] = sum_b part[i][b] in a fixed order (kParts doubles each); if alpha != null,
-// alpha[0] += Re c[j].
-template <int kParts>
-__global__ void k_finish_dots(const double* __restrict__ part, int nv, int nb, double* __restrict__ c,
-                              double* __restrict__ alpha, int j) {
-  __shared__ double red[kVecThreads / 32];
-  for (int i = 0; i < nv; ++i) {
-    for (int r = 0; r < kParts; ++r) {
-      double acc = 0.0;
-      for (int b = threadIdx.x; b < nb; b += blockDim.x) acc += part[((int64_t)i * nb + b) * kParts + r];
-      const double t = block_sum(acc, red);
-      if (threadIdx.x == 0) {
-        c[i * kParts + r] = t;
-        if (alpha && i == j && r == 0) alpha[0] += t;
-      }
-    }
-  }
-}
-
-// w -= sum_i c[i] V_i
-template <class Ops>
-__global__ void __launch_bounds__(kVecThreads) k_subtract(const typename Ops::T* __restrict__ V, int nv, int64_t ld,
-                                                          const double* __restrict__ c, typename Ops::T* __restrict__ w,
-                                                          int64_t n) {
-  __shared__ double cs[64 * Ops::kParts];
-  for (int i = threadIdx.x; i < nv * Ops::kParts; i += blockDim.x) cs[i] = c[i];
-  __syncthreads();
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-    typename Ops::T x = w[e];
-    for (int i = 0; i < nv; ++i) x = Ops::axpy_neg(cs + i * Ops::kParts, __ldg(V + (int64_t)i * ld + e), x);
+    for (int u = 0; u < G; ++u) x = Ops::axpy_neg(k + u * Ops::kParts, v[u], x);
     w[e] = x;
   }
 }
 
-// beta = ||w|| (from the partial sums of squares); v = w / beta (zero vector if beta == 0).
-__global__ void k_finish_norm(const double* __restrict__ part, int nb, double* __restrict__ beta) {
-  __shared__ double red[kVecThreads / 32];
-  double acc = 0.0;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) acc += part[b];
-  const double t = block_sum(acc, red);
-  if (threadIdx.x == 0) beta[0] = sqrt(t);
+// f.template operator()<G>(first vector) over nv vectors in groups of kGroup / kParts
+template <class Ops, typename F>
+__device__ __forceinline__ void by_group(int nv, F&& f) {
+  constexpr int kMost = kGroup / Ops::kParts;
+  int i = 0;
+  for (; i + kMost <= nv; i += kMost) f(std::integral_constant<int, kMost>{}, i);
+  switch (nv - i) {
+    case 1: f(std::integral_constant<int, 1>{}, i); break;
+    case 2: f(std::integral_constant<int, 2>{}, i); break;
+    case 3: f(std::integral_constant<int, 3>{}, i); break;
+    default:
+      if constexpr (kMost > 4) {
+        switch (nv - i) {
+          case 4: f(std::integral_constant<int, 4>{}, i); break;
+          case 5: f(std::integral_constant<int, 5>{}, i); break;
+          case 6: f(std::integral_constant<int, 6>{}, i); break;
+          case 7: f(std::integral_constant<int, 7>{}, i); break;
+          default: break;
+        }
+      }
+  }
+}
+
+// One pass of the Gram-Schmidt step over w, every CTA its own chunk of elements:
+//   SUB:    w -= sum_i c[i] V_i                 (c: the dots of the pass before)
+//   !NORM:  c_out[i] = <V_i, w>;  alpha[0] += Re c_out[j]
+//   NORM:   c_out[0] = ||w||
+// The CTA that finishes last adds the partial sums in CTA order (deterministic). A step is three
+// passes - dots; subtract and dots; subtract and norm - instead of seven launches. Bound by the
+// FP64 pipe (one warp instruction per 32 elements, vector and dot or subtraction).
+// 8 steps on 744k real elements (one two-site vector of D = 2000), launches timed one by one:
+// dots, subtractions, norms and scaling together 950 -> 520 us; the whole run with its matvecs
+// 2800 -> 2400 us.
+template <class Ops, bool SUB, bool NORM>
+__global__ void __launch_bounds__(kVecThreads) k_gram_schmidt(const typename Ops::T* __restrict__ V, int nv, int64_t ld,
+                                                              const double* __restrict__ c_in,
+                                                              typename Ops::T* __restrict__ w, int64_t n,
+                                                              double* __restrict__ part, int* __restrict__ arrived,
+                                                              double* __restrict__ c_out, double* __restrict__ alpha,
+                                                              int j) {
+  using T = typename Ops::T;
+  __shared__ double red[kVecWarps][kGroup];
+  __shared__ int last;
+  const int64_t per = (n + gridDim.x - 1) / gridDim.x;
+  const int64_t e0 = (int64_t)blockIdx.x * per, e1 = min(n, e0 + per);
+  if constexpr (SUB)
+    by_group<Ops>(nv, [&](auto g, int i) {
+      subtract_group<Ops, decltype(g)::value>(V + (int64_t)i * ld, ld, c_in + i * Ops::kParts, w, e0, e1);
+    });
+  // (a thread reads back only elements it wrote itself)
+  int values;
+  if constexpr (NORM) {
+    // |z|^2 = re^2 + im^2: the real dot of the doubles with themselves
+    const double* x = reinterpret_cast<const double*>(w);
+    double acc[1] = {};
+    for (int64_t e = e0 + threadIdx.x; e < e1; e += kVecThreads) {
+#pragma unroll
+      for (int r = 0; r < Ops::kParts; ++r) {
+        const double v = x[e * Ops::kParts + r];
+        acc[0] = fma(v, v, acc[0]);
+      }
+    }
+    const double t = warp_sums<1>(acc, threadIdx.x & 31);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][0] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double s = red[0][0];
+      for (int q = 1; q < kVecWarps; ++q) s += red[q][0];
+      part[blockIdx.x] = s;
+    }
+    values = 1;
+  } else {
+    by_group<Ops>(nv, [&](auto g, int i) {
+      dot_group<Ops, decltype(g)::value>(V + (int64_t)i * ld, ld, w, e0, e1, red,
+                                         part + (int64_t)i * Ops::kParts * gridDim.x);
+    });
+    values = nv * Ops::kParts;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(arrived, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  if (threadIdx.x == 0) *arrived = 0;   // for the next launch
+  __threadfence();
+  const int lane = threadIdx.x & 31;
+  for (int i = threadIdx.x >> 5; i < values; i += kVecWarps) {
+    double v[1] = {};
+    for (int b = lane; b < (int)gridDim.x; b += 32) v[0] += __ldcg(part + (int64_t)i * gridDim.x + b);
+    const double t = warp_sums<1>(v, lane);
+    if (lane == 0) {
+      c_out[i] = NORM ? sqrt(t) : t;
+      if (!NORM && i == j * Ops::kParts) alpha[0] += t;
+    }
+  }
 }
 
 __global__ void __launch_bounds__(kVecThreads) k_scale_into(const double* __restrict__ w,
@@ -188,8 +253,8 @@ struct qltg_lanczos {
   int64_t n = 0;          // elements of ψ
   int64_t ld = 0;         // stride between Krylov vectors in elements (n rounded up to 32)
   int steps = 0;          // steps taken since the last start
-  // coef: alpha[max_iter] | beta[max_iter + 1] | c[2 (max_iter + 1)]
-  DevBuf V, w, part, coef;
+  // coef: alpha[max_iter] | beta[max_iter + 1] | c[2 (max_iter + 1)] | the second pass's c
+  DevBuf V, w, part, coef, arrived;
   std::vector<cudaGraphExec_t> graphs;
   std::vector<cudaGraph_t> graph_defs;
   cudaStream_t capture = nullptr;
@@ -198,7 +263,8 @@ struct qltg_lanczos {
   int64_t n_doubles() const { return n * parts(); }
   double* alpha() const { return coef.as<double>(); }
   double* beta() const { return coef.as<double>() + max_iter; }
-  double* cbuf() const { return coef.as<double>() + 2 * max_iter + 1; }
+  double* cbuf(int pass) const { return coef.as<double>() + 2 * max_iter + 1 + pass * 2 * (max_iter + 1); }
+  int64_t coef_doubles() const { return 2 * max_iter + 1 + 4 * (int64_t)(max_iter + 1); }
   double* vec(int i) const { return V.as<double>() + (int64_t)i * ld * parts(); }
 
   ~qltg_lanczos() {
@@ -209,23 +275,23 @@ struct qltg_lanczos {
     if (capture) cudaStreamDestroy(capture);
   }
 
+  // two passes of classical Gram-Schmidt of w against v_0 .. v_j, then beta_{j+1} = ||w||
   template <class Ops>
   void gram_schmidt(int j, cudaStream_t s) {
     using T = typename Ops::T;
     const T* Vt = V.as<T>();
     T* wt = w.as<T>();
-    for (int pass = 0; pass < 2; ++pass) {
-      k_multi_dot<Ops><<<kVecBlocks, kVecThreads, 0, s>>>(Vt, j + 1, ld, wt, n, part.as<double>());
-      k_finish_dots<Ops::kParts><<<1, kVecThreads, 0, s>>>(part.as<double>(), j + 1, kVecBlocks, cbuf(),
-                                                           alpha() + j, j);
-      k_subtract<Ops><<<kVecBlocks, kVecThreads, 0, s>>>(Vt, j + 1, ld, cbuf(), wt, n);
-    }
+    double* pt = part.as<double>();
+    int* arr = arrived.as<int>();
+    k_gram_schmidt<Ops, false, false><<<kVecBlocks, kVecThreads, 0, s>>>(Vt, j + 1, ld, nullptr, wt, n, pt, arr, cbuf(0), alpha() + j, j);
+    k_gram_schmidt<Ops, true, false><<<kVecBlocks, kVecThreads, 0, s>>>(Vt, j + 1, ld, cbuf(0), wt, n, pt, arr, cbuf(1), alpha() + j, j);
+    k_gram_schmidt<Ops, true, true><<<kVecBlocks, kVecThreads, 0, s>>>(Vt, j + 1, ld, cbuf(1), wt, n, pt, arr, beta() + j + 1, nullptr, 0);
   }
 
-  // ||x||: the real multi-dot of x with itself over its doubles (|z|^2 = re^2 + im^2)
+  // ||x|| of n_doubles() values (x is only read)
   void norm_into(const double* x, double* out, cudaStream_t s) {
-    k_multi_dot<RealOps><<<kVecBlocks, kVecThreads, 0, s>>>(x, 1, 0, x, n_doubles(), part.as<double>());
-    k_finish_norm<<<1, kVecThreads, 0, s>>>(part.as<double>(), kVecBlocks, out);
+    k_gram_schmidt<RealOps, false, true><<<kVecBlocks, kVecThreads, 0, s>>>(
+        nullptr, 0, 0, nullptr, const_cast<double*>(x), n_doubles(), part.as<double>(), arrived.as<int>(), out, nullptr, 0);
   }
 
   // the kernels of step j, enqueued on s
@@ -233,7 +299,6 @@ struct qltg_lanczos {
     mv->enqueue(vec(j), w.get(), s);
     if (cplx) gram_schmidt<ComplexOps>(j, s);
     else gram_schmidt<RealOps>(j, s);
-    norm_into(w.as<double>(), beta() + j + 1, s);
     k_scale_into<<<kVecBlocks, kVecThreads, 0, s>>>(w.as<double>(), beta() + j + 1, vec(j + 1), n_doubles());
   }
 };
@@ -257,10 +322,13 @@ int qltg_lanczos_create(qltg_matvec* mv, int32_t max_iter, qltg_lanczos** lz) {
     h->V.alloc(std::max<int64_t>(1, (int64_t)(max_iter + 1) * h->ld) * eb);
     h->w.alloc(std::max<int64_t>(1, h->ld) * eb);
     h->part.alloc((int64_t)kVecBlocks * (max_iter + 1) * 2 * 8);
-    h->coef.alloc((int64_t)(4 * max_iter + 3) * 8);
+    h->coef.alloc(h->coef_doubles() * 8);
+    h->arrived.alloc(sizeof(int));
     h->graphs.assign(max_iter, nullptr);
     h->graph_defs.assign(max_iter, nullptr);
     QLTG_CUDA(cudaStreamCreateWithFlags(&h->capture, cudaStreamNonBlocking));
+    QLTG_CUDA(cudaMemsetAsync(h->arrived.get(), 0, sizeof(int), h->capture));
+    QLTG_CUDA(cudaStreamSynchronize(h->capture));   // before any stream runs a step
     *lz = h.release();
   });
 }
@@ -270,7 +338,7 @@ int qltg_lanczos_start(qltg_lanczos* lz, const void* psi0_dev, void* stream) {
     QLTG_CHECK(lz && psi0_dev, QLTG_ERR_INVALID, "null Lanczos or psi0");
     QLTG_CUDA(cudaSetDevice(lz->mv->ctx->device));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    k_zero<<<1, kVecThreads, 0, s>>>(lz->coef.as<double>(), 4 * lz->max_iter + 3);
+    k_zero<<<1, kVecThreads, 0, s>>>(lz->coef.as<double>(), (int)lz->coef_doubles());
     const double* x = static_cast<const double*>(psi0_dev);
     lz->norm_into(x, lz->beta(), s);   // beta_0 = ||psi0||
     k_scale_into<<<kVecBlocks, kVecThreads, 0, s>>>(x, lz->beta(), lz->vec(0), lz->n_doubles());

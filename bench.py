@@ -14,7 +14,7 @@ e2e    : the same through the public API with host buffers (qltg_matvec_apply_ho
          host psi copied in, H_eff psi computed, result copied back - every step.
 roofline: the dominant kernel (grouped GEMM) timed with CUDA events on its own stream:
          algorithmic FP64 flops sum(2mkn) / launch time against the FP64-equivalent peak
-         (split: the BF16 peak / 28 slice products; FP64: cuBLAS DGEMM measured in the run);
+         (split: the BF16 peak / 21 slice products; FP64: cuBLAS DGEMM measured in the run);
          sum_T_over_t = sum over the four steps of max(F/P, B/BW) / the matvec time.
 cpu_baseline: the CPU restatement of the reference's algorithm (OpenBLAS dgemm per block
          pair, as the reference's CPU build) on a bounded sample of the same workload.
@@ -38,6 +38,8 @@ sys.path.insert(0, ROOT)
 WORKLOAD = dict(D=4000, qmax=30, sigma=9.0, seed=1)
 WORKLOAD_NAME = "two-site H*psi matvec, U(1) Heisenberg chain, D=4000 (Sz -30..30, sigma 9), d=2, w=5"
 METRIC = "two-site H*psi matvec s/iter at D=4000"
+# split precision: slice products per FP64 product, and the k extent that the plan counts tiles in
+SPLIT_PAIRS, SPLIT_STAGE_K = 21, 32
 L2_FLUSH_BYTES = 512 << 20
 
 
@@ -246,9 +248,9 @@ def gemm_roofline(mode, lenv, psi, d1, d2, dr, dl, dp, local, stream, flush, pk)
         f, _ = p.stats()
         tcf, useful = 0.0, None
         if mode == "split":
-            # 28 slice pairs on 128 x 32 x 32 tile stages (padding included), as scheduled
+            # every slice pair of the 128 x 32 x SPLIT_STAGE_K tile stages (padding included), as scheduled
             stages, useful = p.split_stats()
-            tcf = stages * 28 * (2 * 128 * 32 * 32)
+            tcf = stages * SPLIT_PAIRS * (2 * 128 * 32 * SPLIT_STAGE_K)
         sch = p.schedule()
         per.append({"transpose_ms": round(ms1, 4), "stage_ms": round(ms2, 4), "kernel_ms": round(ms3, 4),
                     "gflop": round(f / 1e9, 4),
@@ -265,19 +267,19 @@ def gemm_roofline(mode, lenv, psi, d1, d2, dr, dl, dp, local, stream, flush, pk)
     i, ms, work, f = best
     exec_tflops = exec_frac = None
     if mode == "split":
-        # the slice-pipe peak divided by the 28 slice products each FP64 product needs
+        # the slice-pipe peak divided by the slice products each FP64 product needs
         bf16 = pk["bf16_tflops"]
-        peak = bf16 / 28.0
-        src = (f"bf16 dense burst {bf16:.1f} TFLOP/s ({pk['source']}, MEASURED_PEAKS.json) / 28 slice "
+        peak = bf16 / SPLIT_PAIRS
+        src = (f"bf16 dense burst {bf16:.1f} TFLOP/s ({pk['source']}, MEASURED_PEAKS.json) / {SPLIT_PAIRS} slice "
                "products = the FP64-equivalent peak of the split form")
         what = (f"k_gemm_split, one launch (matvec step {i}): algorithmic FP64 flops sum(2mkn) / launch time, "
-                "against the BF16 peak / 28")
+                f"against the BF16 peak / {SPLIT_PAIRS}")
         exec_tflops = work / (ms / 1e3) / 1e12
         exec_frac = exec_tflops / bf16
     else:
         peak = fp64_peak_tflops(local, stream)
         src = "cuBLAS DGEMM 8192^3 measured in this run (the FP64 pipe)"
-        what = f"k_gemm_dfma (+ k_gemm_skinny), one launch (matvec step {i}): algorithmic flops sum(2mkn) / launch time"
+        what = f"k_gemm_f64 (+ k_gemm_skinny), one launch (matvec step {i}): algorithmic flops sum(2mkn) / launch time"
     achieved = f / (ms / 1e3) / 1e12
     # whole-matvec bound: per step T_s = max(F_s / P, B_s / BW)
     bw = pk["hbm_gbs"] * 1e9
@@ -294,7 +296,8 @@ def gemm_roofline(mode, lenv, psi, d1, d2, dr, dl, dp, local, stream, flush, pk)
     if exec_tflops is not None:
         out["executed_tensor_tflops"] = exec_tflops
         out["executed_tensor_frac"] = exec_frac
-        out["executed_note"] = "executed BF16 tensor flops (28 slice pairs on 128x32x32 padded tiles) / launch time / BF16 peak"
+        out["executed_note"] = (f"executed BF16 tensor flops ({SPLIT_PAIRS} slice pairs on 128x32x{SPLIT_STAGE_K} padded tiles) "
+                                "/ launch time / BF16 peak")
     return out
 
 
@@ -663,8 +666,8 @@ def run_aux(local: int, part: str = "all"):
         ms = _time_events(lambda: mv.apply(dp_, o), stream, flush, reps=10)
         mv.device_status()
         f, _ = mv.stats()
-        # 8(d): P = FP64 pipe (fp64) or BF16 peak / 28 slice products (split), BW = HBM
-        peak = fp64_peak_tflops(local, stream) if mode == "fp64" else pk["bf16_tflops"] / 28.0
+        # 8(d): P = FP64 pipe (fp64) or BF16 peak / slice products (split), BW = HBM
+        peak = fp64_peak_tflops(local, stream) if mode == "fp64" else pk["bf16_tflops"] / SPLIT_PAIRS
         _, t_bound = matvec_step_bounds(tensors, local, peak, pk["hbm_gbs"])
         r = {"mode": mode, "ms": round(ms, 4), "gflops": f / (ms / 1e3) / 1e9, "plan_s": round(t_create, 3),
              "schedules": mv.schedules(),

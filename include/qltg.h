@@ -51,9 +51,9 @@ enum { QLTG_IN = 0, QLTG_OUT = 1 };       /* TenIndexDirType */
 /* Arithmetic of a contraction.
  * QLTG_MODE_FP64:  plain FP64 on the FP64 pipe, the reference's precision.
  * QLTG_MODE_SPLIT: FP64 emulated with BF16 slices on the tcgen05 tensor cores: every row
- *                  of A / column of B is scaled by a power of two and cut into seven 7-bit
- *                  integer slices, the 28 slice products of weight >= 2^-56 accumulate
- *                  exactly (FP32 integers in tensor memory, drained every 256 k into int64),
+ *                  of A / column of B is scaled by a power of two and rounded to six
+ *                  balanced 8-bit digits, the 21 slice products of weight >= 2^-56 accumulate
+ *                  exactly (FP32 integers in tensor memory, drained every 160 k into int64),
  *                  and each task's sum is rounded to FP64 once. Per element the error is
  *                  below 2^-48 * sum_k |a_ik| |b_kj| scaled by the row / column maxima
  *                  (about 1e-14 relative for random data); the tests and the benchmark

@@ -5,18 +5,25 @@
 // Slicing (per operand block, integer arithmetic only - the FP64 pipe of this GPU runs at
 // about 1 TFLOP/s, so nothing on the hot path leans on it):
 //   every row i of A (column j of B) gets a scale 2^e with max |x| < 2^e, and each element
-//   x = s 2^e y, |y| < 1, is cut into S = 7 base-2^7 digits of Y = floor(|y| 2^49):
-//   x ~= 2^e sum_p a_p 2^(-7p), digits a_p = s d_p in [-127, 127]. Slice p is stored as
-//   the BF16 number a_p 2^(-7p) (exact: 7 significant bits). Truncation error < 2^-49 of
-//   the row (column) maximum.
-// Products (the Ozaki scheme, restated): C_ij = 2^(ea_i + eb_j) sum over the 28 slice pairs
-//   p + q <= 8 of (A_p B_q)_ij. Level L = p + q sums L - 1 pairs, each an integer multiple
-//   of 2^(-7L) below 2^14 of those units. Each level has its own 128 x 32 FP32 accumulator
-//   in tensor memory (levels 2..8: 224 columns per set, two sets). Over 256 k the sums of
-//   levels 2..5 stay below 2^24 and are exact; levels 6..8 may round in FP32, at most
-//   2^-24 of a quantity 2^-28 below the leading level. Every 256 k the drain warps read the
-//   levels and fold them into one int64 per output (units 2^-49); at the end of a task
-//   C (+)= sign 2^(ea + eb - 49) z, rounded to FP64 with integer operations.
+//   x = s 2^e y, |y| < 1, is rounded to Y = round(|y| 2^48) and written in S = 6 balanced
+//   base-2^8 digits: x ~= 2^e sum_p a_p 2^(-8p), a_p = s d_p with d_1 in [0, 256] and
+//   d_2 .. d_6 in [-128, 127]. Slice p is stored as the BF16 number a_p 2^(-8p) (exact: a
+//   BF16 significand has 8 bits, and 256 is a power of two). Rounding error <= 2^-49 of the
+//   row (column) maximum. Balanced digits use all 8 bits and the sign of a BF16 number, so six
+//   slices hold what seven slices of 7-bit digits of one sign do, and 21 products suffice where
+//   those need 28; the error against 64-bit products is 3-4 times smaller (rounding instead of
+//   truncation; the level left out, 8, has rms 2^-50.4 of the maxima, 7-bit level 9 2^-49.3).
+// Products (the Ozaki scheme, restated): C_ij = 2^(ea_i + eb_j) sum over the 21 slice pairs
+//   p + q <= 7 of (A_p B_q)_ij. Level L = p + q sums L - 1 pairs, each an integer multiple of
+//   2^(-8L) of at most 2^16 (L = 2), 2^15 (a first digit) or 2^14 of those units. Each level
+//   has its own 128 x 32 FP32 accumulator in tensor memory (levels 2..7: 192 columns per set,
+//   two sets). Over 160 k the sums of levels 2..5 stay below 2^24 (level 5: 160 x 3 x 2^15) and
+//   are exact; level 6 may pass 2^24 by 1.1 and level 7 by 1.25 where every digit is at its
+//   limit, and then carry an FP32 rounding of one unit, 2^-48 or 2^-56. Every 160 k the drain
+//   warps read the levels and fold them into one int64 per output (units 2^-51); at the end of
+//   a task C (+)= sign 2^(ea + eb - 51) z, rounded to FP64 with integer operations.
+// D = 4000 matvec: k_gemm_split 122 / 97 -> 98 / 90 us (steps 0 / 3), k_pack_a 55 -> 48 us; error
+// against 64 bits 1.2e-13 -> 2.5e-14.
 //
 // Layout for the tensor cores: both operands K-major, no swizzle, in 8 x 16-byte core
 // matrices (leading-byte offset 128 B between the two core matrices of a 16-wide k step,
@@ -26,7 +33,7 @@
 //
 // GEMM: one persistent CTA per SM, warp-specialised (see k_gemm_split): a producer warp
 // streams 32-wide k slabs of all A and B slices into shared memory, an MMA warp issues per
-// 16-wide k step 7 MMAs (A slice p against B slices 1..8-p concatenated along N), sixteen
+// 16-wide k step 6 MMAs (A slice p against B slices 1..7-p concatenated along N), sixteen
 // drain warps fold the accumulators. Output rows reach C through a row map, so the A blocks
 // of several output blocks can share one 128-row tile (row stacking).
 // Every wait on an mbarrier is bounded; on expiry the CTA sets the plan's error word,
@@ -45,12 +52,13 @@
 namespace qltg {
 namespace {
 
-constexpr int kS = 7;                      // slices
-constexpr int kLevels = 7;                 // accumulators: levels 2..8
+constexpr int kS = 6;                      // slices
+constexpr int kLevels = 6;                 // accumulators: levels 2..7
+constexpr int kUnit = 51;                  // the int64 sums are in units of 2^-kUnit
 constexpr int kTM = 128, kTN = 32, kTK = 64;
 constexpr int kATile = kTM * kTK * 2;      // bytes of one (row tile, k tile, slice): 16 KB
 constexpr int kBTile = kTN * kTK * 2;      // 4 KB
-constexpr int kDrainK = 256;               // k between drains (exactness bound of levels 2..5)
+constexpr int kDrainK = 160;               // k between drains (exactness bound of levels 2..5)
 
 // ------------------------------------------------------------------ slicing
 // Work distribution of the slicing kernels: CTA b takes the contiguous item range
@@ -66,10 +74,13 @@ __device__ __forceinline__ int field_of_bits(uint64_t absbits) {
 }
 __device__ __forceinline__ int exp_of_field(int f) { return f ? f - 1022 : 0; }
 
-// |x| / 2^e as the 49-bit integer Y = floor(|x| 2^(49 - e)) and the sign as a BF16 sign bit,
-// in 32-bit halves: Y = (hidden bit : fraction) >> sh with sh = 1026 + e - max(ex, 1) >= 4
-// (|x| < 2^e); zero has no hidden bit and a zero fraction, so it gives Y = 0.
-__device__ __forceinline__ uint64_t scaled_y(double x, int e, uint32_t& sgn) {
+// The digits of |x| / 2^e and the sign of x as a BF16 sign bit, in 32-bit halves. The result is
+// Y + the bias 128 (2^32 + 2^24 + 2^16 + 2^8 + 1), Y = round(|x| 2^(48 - e)) (ties up): bits
+// 40 .. 48 are the first digit, and byte 6 - p, less 128, is digit p = 2 .. 6. One bit more than
+// Y comes from (hidden bit : fraction) >> sh, with sh = 1026 + e - max(ex, 1) >= 4
+// (|x| < 2^e); half an ulp and the bias (doubled) are added to it at once. Zero has no hidden
+// bit and a zero fraction: all its digits are 0.
+__device__ __forceinline__ uint64_t digits_of(double x, int e, uint32_t& sgn) {
   const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
   sgn = (hi >> 16) & 0x8000u;
   const uint32_t ex = (hi >> 20) & 0x7FFu;
@@ -78,31 +89,28 @@ __device__ __forceinline__ uint64_t scaled_y(double x, int e, uint32_t& sgn) {
   const bool small = sh < 32;
   const uint32_t yl = small ? __funnelshift_r(lo, mhi, sh) : (mhi >> min(sh - 32, 31));
   const uint32_t yh = small ? (mhi >> sh) : 0u;
-  return ((uint64_t)yh << 32) | yl;
+  const uint64_t t = (((uint64_t)yh << 32) | yl) + 0x0000010101010101ull;
+  return t >> 1;
 }
-// Slice p of two elements as one word of two BF16 values: digit d = bits 7 (kS - 1 - p) ..
-// + 6 of Y, value d 2^(-7(p+1)) with the element's sign. The digit is or-ed into the
-// mantissa of 2^23 (float 2^23 + d), one FMA scales and removes the 2^23 exactly (d has at
-// most 7 significant bits, so the float's low 16 bits are zero and its high half is the
-// exact BF16), one byte permute takes both high halves.
+// Slice P + 1 of two elements as one word of two BF16 values: the digit's byte (the first
+// digit: bytes 5 and 6) goes into the mantissa of 2^23 by one byte permute (float 2^23 + b), one
+// FMA removes 2^23 and the bias and scales, exactly (a digit has at most 8 significant bits, so
+// the float's low 16 bits are zero and its high half is the exact BF16), one byte permute takes
+// both high halves; the elements' signs are xor-ed in.
 template <int P>
-__device__ __forceinline__ uint32_t digit_magic(uint64_t y) {
-  const uint32_t hi = (uint32_t)(y >> 32), lo = (uint32_t)y;
-  constexpr int sh = 7 * (kS - 1 - P);
-  uint32_t x;
-  if constexpr (sh >= 32) x = hi >> (sh - 32);
-  else if constexpr (sh + 7 > 32) x = __funnelshift_r(lo, hi, sh);
-  else x = lo >> sh;
-  return (x & 127u) | 0x4B000000u;
+__device__ __forceinline__ float digit_value(uint64_t y) {
+  constexpr uint32_t bits = (uint32_t)(127 - 8 * (P + 1)) << 23;
+  const uint32_t word = P < 2 ? (uint32_t)(y >> 32) : (uint32_t)y;
+  constexpr uint32_t sel = P == 0 ? 0x7621u : 0x7540u | (uint32_t)(P == 1 ? 0 : kS - 1 - P);
+  const float scale = __uint_as_float(bits);
+  const float bias = P == 0 ? 8388608.0f : 8388608.0f + 128.0f;
+  return __fmaf_rn(__uint_as_float(__byte_perm(word, 0x4B000000u, sel)), scale, -bias * scale);
 }
 template <int P>
 __device__ __forceinline__ uint32_t plane_pair(uint64_t y0, uint64_t y1, uint32_t sgn_pair) {
-  const float scale = __uint_as_float((uint32_t)(127 - 7 * (P + 1)) << 23);
-  const float f0 = __fmaf_rn(__uint_as_float(digit_magic<P>(y0)), scale, -8388608.0f * scale);
-  const float f1 = __fmaf_rn(__uint_as_float(digit_magic<P>(y1)), scale, -8388608.0f * scale);
-  return __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632) | sgn_pair;
+  return __byte_perm(__float_as_uint(digit_value<P>(y0)), __float_as_uint(digit_value<P>(y1)), 0x7632) ^ sgn_pair;
 }
-// The 7 slice planes of 8 consecutive elements, written as 16-byte words at dst + p stride.
+// The 6 slice planes of 8 consecutive elements, written as 16-byte words at dst + p stride.
 __device__ __forceinline__ void store_planes(const uint64_t* y, const uint32_t* sg, uint8_t* dst, int stride) {
   const uint32_t s01 = sg[0] | (sg[1] << 16), s23 = sg[2] | (sg[3] << 16), s45 = sg[4] | (sg[5] << 16),
                  s67 = sg[6] | (sg[7] << 16);
@@ -115,7 +123,7 @@ __device__ __forceinline__ void store_planes(const uint64_t* y, const uint32_t* 
     v.w = plane_pair<P>(y[6], y[7], s67);                                                       \
     *reinterpret_cast<uint4*>(dst + P * stride) = v;                                            \
   }
-  QLTG_PLANE(0) QLTG_PLANE(1) QLTG_PLANE(2) QLTG_PLANE(3) QLTG_PLANE(4) QLTG_PLANE(5) QLTG_PLANE(6)
+  QLTG_PLANE(0) QLTG_PLANE(1) QLTG_PLANE(2) QLTG_PLANE(3) QLTG_PLANE(4) QLTG_PLANE(5)
 #undef QLTG_PLANE
 }
 
@@ -255,8 +263,8 @@ __global__ void __launch_bounds__(256) k_pack_a(const double* __restrict__ scr, 
     // the row's place in its stacked operand: 128-row tile vt, row vr inside it
     const int vrow = o.row_base + (int)row;
     const int vt = vrow / kTM, vr = vrow - vt * kTM;
-    // tile layout [ks][slice][m_core][k_core][8 rows x 16 B]: the 7 slices of a 16-wide k
-    // step are contiguous, so a 32-wide stage is one 56 KB copy
+    // tile layout [ks][slice][m_core][k_core][8 rows x 16 B]: the slices of a 16-wide k step
+    // are contiguous, so a 32-wide stage is one 48 KB copy
     const int kt = k0 / kTK, ks = (k0 % kTK) >> 4;
     const int64_t tile = (int64_t)vt * o.ktiles + kt;
     uint8_t* dst = pack + o.pack_off + tile * (int64_t)(kS * kATile) + (int64_t)ks * (kS * 4096) + (vr >> 3) * 256 +
@@ -268,7 +276,7 @@ __global__ void __launch_bounds__(256) k_pack_a(const double* __restrict__ scr, 
       uint64_t y[8];
       uint32_t sg[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) y[j] = scaled_y((kb + j < o.cols) ? __ldg(src_row + kb + j) : 0.0, e, sg[j]);
+      for (int j = 0; j < 8; ++j) y[j] = digits_of((kb + j < o.cols) ? __ldg(src_row + kb + j) : 0.0, e, sg[j]);
       store_planes(y, sg, dst + half * 128, 4096);
     }
   }
@@ -356,10 +364,10 @@ __global__ void __launch_bounds__(256) k_pack_b_cols(const double* __restrict__ 
           if constexpr (CPLX) x = b_elem<true>(blk, k0 + j, c0 + cc, o.cols);
           else x = col[(k0 + j) * o.cols];
         }
-        y[j] = scaled_y(x, e, sg[j]);
+        y[j] = digits_of(x, e, sg[j]);
       }
-      // tile layout [ks][slice][n_core][k_core][8 columns x 16 B]: the 7 slices of a 16-wide k
-      // step form one 224-row K-major operand (slice q = rows 32 (q-1) .. 32 q - 1)
+      // tile layout [ks][slice][n_core][k_core][8 columns x 16 B]: the slices of a 16-wide k
+      // step form one 192-row K-major operand (slice q = rows 32 (q-1) .. 32 q - 1)
       const int64_t tile = (int64_t)tt.y * o.ktiles + kt;
       store_planes(y, sg, pack + o.pack_off + tile * (int64_t)(kS * kBTile) + (int64_t)ks * (kS * 1024) + n_core * 256 +
                               k_core * 128 + n8 * 16, 1024);
@@ -386,30 +394,29 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int n) {
 // checking the clock every 256 polls so the fast path is a bare try_wait.
 constexpr long long kWaitCycles = 1ll << 31;
 
-// Operand pipeline: a stage holds one 32-wide k slab of all 7 A slices (56 KB) and all 7 B
-// slices (14 KB), each as it lies in the packed tile ([16-wide k step][slice][...]); 3
-// stages = 210 KB of shared memory. Per 16-wide k step the A slices are 4 KB apart and the
-// B slices form one 224-row operand.
+// Operand pipeline: a stage holds one 32-wide k slab of all A slices (48 KB) and all B slices
+// (12 KB), each as it lies in the packed tile ([16-wide k step][slice][...]); 3 stages = 180 KB
+// of shared memory. Per 16-wide k step the A slices are 4 KB apart and the B slices form one
+// 192-row operand.
 constexpr int kStages = 3;
 constexpr int kKS = 32;                         // k per stage (2 MMA k-steps)
-constexpr int kAStep = kS * kTM * 16 * 2;       // 28 KB: 7 A slices of one k step
-constexpr int kBStep = kS * kTN * 16 * 2;       // 7 KB: 7 B slices of one k step
+constexpr int kAStep = kS * kTM * 16 * 2;       // 24 KB: the A slices of one k step
+constexpr int kBStep = kS * kTN * 16 * 2;       // 6 KB: the B slices of one k step
 constexpr int kABytes = 2 * kAStep, kBBytes = 2 * kBStep;
-constexpr int kStageBytes = kABytes + kBBytes;  // 70 KB
+constexpr int kStageBytes = kABytes + kBBytes;  // 60 KB
 constexpr int kSmemBytes = kStages * kStageBytes + 1024;
-constexpr int kPeriod = kDrainK / kKS;          // stages between drains (4)
+constexpr int kPeriod = kDrainK / kKS;          // stages between drains (5)
 constexpr int kDrainWarps = 16;                 // four per tensor-memory lane quadrant
 constexpr int kDrainCols = kTN / 4;             // columns per drain thread
 constexpr int kRoleThreads = 64 + 32 * kDrainWarps;   // warp 0 producer, warp 1 MMA, warps 2-17 drain
-// Tensor memory: two accumulator sets, each 7 levels x 32 columns (level L at 32 (L - 2)).
-constexpr int kAccCols = kLevels * kTN;         // 224
+// Tensor memory: two accumulator sets, each 6 levels x 32 columns (level L at 32 (L - 2)).
+constexpr int kAccCols = kLevels * kTN;         // 192
 // Then the tile's running FP64 sum over its tasks: 32 doubles per lane as 64 32-bit columns.
-constexpr int kSumCol = 2 * kAccCols;           // 448
+constexpr int kSumCol = 2 * kAccCols;           // 384
 constexpr uint32_t kTmemAlloc = 512;
+static_assert(kDrainK % kKS == 0, "whole stages between drains");
 static_assert(kSumCol + 2 * kTN <= (int)kTmemAlloc, "tensor memory budget");
-constexpr int kFlushDrains = 32;                // the int64 sum of a chunk stays below 2^63
-constexpr float kMagic = 12582912.0f;           // 1.5 * 2^23: x + kMagic has the integer x in its low bits
-constexpr int kMagicBits = 0x4B400000;          // for |x| < 2^22
+constexpr int kFlushDrains = 12;                // the int64 sum of 12 x 160 k stays below 2^62
 
 __device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count));
@@ -521,51 +528,39 @@ __global__ void __launch_bounds__(32) k_wait_selftest(long long limit, int* __re
   if (threadIdx.x == 0) *status = ok ? 0 : 1;
 }
 
-// Fold one drained accumulator set into the int64 sums z (units 2^-49) of this thread's
-// row and 8 columns. Over 256 k, level L sums (L - 1) slice pairs of 256 products below
-// 127^2 each, integers times 2^(-7L): levels 2..5 stay below 2^24 and are exact in FP32;
-// levels 6..8 may pass 2^24 and carry an FP32 rounding there, at most 2^-24 of a quantity
-// 2^-28 below the leading level (2^-52 of the result: below the 2^-49 slice truncation).
-// Level 2 stays below 2^22 and converts with the magic-number add, the others with F2I;
-// level 8 is rounded to units of 2^-49.
+// Fold one drained accumulator set into the int64 sums z (units 2^-51) of this thread's row
+// and 8 columns. Level L holds integers times 2^(-8L), each below 2^24.4 over 160 k (see the
+// head of this file), so F2I gives them as they are; level 7 is rounded to units of 2^-51.
+// Level 2's units reach the high word only.
 __device__ __forceinline__ void drain_set(uint32_t lb, long long (&z)[kDrainCols]) {
   // levels are read two at a time, one wait per pair
   uint32_t r[kDrainCols], q[kDrainCols];
-  int32_t u[kDrainCols];
   tmem_ld8(lb, r);                                       // level 2
   tmem_ld8(lb + kTN, q);                                 // level 3
   asm volatile("tcgen05.wait::ld.sync.aligned;");
 #pragma unroll
   for (int c = 0; c < kDrainCols; ++c) {
-    u[c] = (__float_as_int(fmaf(__uint_as_float(r[c]), 0x1p14f, kMagic)) - kMagicBits) * 128;
-    u[c] += __float2int_rn(__uint_as_float(q[c]) * 0x1p21f);
-    z[c] += (long long)u[c] << 28;
+    const uint32_t h = (uint32_t)__float2int_rn(__uint_as_float(r[c]) * 0x1p19f);   // units 2^-19
+    z[c] += (long long)((uint64_t)h << 32);
+    z[c] += (long long)__float2int_rn(__uint_as_float(q[c]) * 0x1p24f) * (1ll << 27);
   }
   tmem_ld8(lb + 2 * kTN, r);                             // level 4
   tmem_ld8(lb + 3 * kTN, q);                             // level 5
   asm volatile("tcgen05.wait::ld.sync.aligned;");
 #pragma unroll
   for (int c = 0; c < kDrainCols; ++c) {
-    u[c] = __float2int_rn(__uint_as_float(r[c]) * 0x1p28f) * 128;
-    u[c] += __float2int_rn(__uint_as_float(q[c]) * 0x1p35f);
-    z[c] += (long long)u[c] << 14;
+    z[c] += (long long)__float2int_rn(__uint_as_float(r[c]) * 0x1p32f) * (1ll << 19);
+    z[c] += (long long)__float2int_rn(__uint_as_float(q[c]) * 0x1p40f) * (1ll << 11);
   }
-  tmem_ld8(lb + 4 * kTN, r);                             // level 6 (in int64: it may pass 2^24)
+  tmem_ld8(lb + 4 * kTN, r);                             // level 6
   tmem_ld8(lb + 5 * kTN, q);                             // level 7
   asm volatile("tcgen05.wait::ld.sync.aligned;");
 #pragma unroll
-  for (int c = 0; c < kDrainCols; ++c) {
-    z[c] += (long long)__float2int_rn(__uint_as_float(r[c]) * 0x1p42f) * 128;
-    u[c] = __float2int_rn(__uint_as_float(q[c]) * 0x1p49f);
-  }
-  tmem_ld8(lb + 6 * kTN, r);                             // level 8
-  asm volatile("tcgen05.wait::ld.sync.aligned;");
-#pragma unroll
   for (int c = 0; c < kDrainCols; ++c)
-    z[c] += (long long)(u[c] + ((__float2int_rn(__uint_as_float(r[c]) * 0x1p56f) + 64) >> 7));
+    z[c] += (long long)(__float2int_rn(__uint_as_float(r[c]) * 0x1p51f) + __float2int_rn(__uint_as_float(q[c]) * 0x1p51f));
 }
 
-// sum (+)= sign 2^(ea + eb - 49) z, each term rounded once to FP64; the tile's running sum
+// sum (+)= sign 2^(ea + eb - 51) z, each term rounded once to FP64; the tile's running sum
 // of this thread's 8 columns lives in tensor memory at tsum (16 columns). The first
 // contribution to a tile sets it, later ones add.
 __device__ __forceinline__ void fold_sums(const long long (&z)[kDrainCols], int ea, const int (&eb)[kDrainCols],
@@ -576,14 +571,14 @@ __device__ __forceinline__ void fold_sums(const long long (&z)[kDrainCols], int 
     asm volatile("tcgen05.wait::ld.sync.aligned;");
 #pragma unroll
     for (int c = 0; c < kDrainCols; ++c) {
-      const double x = scaled_i64(z[c], ea + eb[c] - 49, neg) + __hiloint2double((int)v[2 * c + 1], (int)v[2 * c]);
+      const double x = scaled_i64(z[c], ea + eb[c] - kUnit, neg) + __hiloint2double((int)v[2 * c + 1], (int)v[2 * c]);
       v[2 * c] = (uint32_t)__double2loint(x);
       v[2 * c + 1] = (uint32_t)__double2hiint(x);
     }
   } else {
 #pragma unroll
     for (int c = 0; c < kDrainCols; ++c) {
-      const double x = scaled_i64(z[c], ea + eb[c] - 49, neg);
+      const double x = scaled_i64(z[c], ea + eb[c] - kUnit, neg);
       v[2 * c] = (uint32_t)__double2loint(x);
       v[2 * c + 1] = (uint32_t)__double2hiint(x);
     }
@@ -599,15 +594,15 @@ __device__ __forceinline__ void fold_sums(const long long (&z)[kDrainCols], int 
 // talking:
 //  * warp 0 fills shared-memory stage g % 3 with two bulk copies once the MMAs of stage
 //    g - 3 released it;
-//  * warp 1 issues, per 16-wide k step, 7 MMAs into accumulator set (period d) % 2 once
-//    the drain warps released it: MMA p multiplies A slice p by B slices 1..8-p
-//    concatenated along N (N = 32 (8 - p)) into the levels p+1..8, i.e. accumulator
-//    columns 32 (p - 1) .. 223, so every slice pair with p + q <= 8 lands on its level
-//    with no padding and the tensor core sees few wide instructions instead of 28 narrow
+//  * warp 1 issues, per 16-wide k step, 6 MMAs into accumulator set (period d) % 2 once
+//    the drain warps released it: MMA p multiplies A slice p by B slices 1..7-p
+//    concatenated along N (N = 32 (7 - p)) into the levels p+1..7, i.e. accumulator
+//    columns 32 (p - 1) .. 191, so every slice pair with p + q <= 7 lands on its level
+//    with no padding and the tensor core sees few wide instructions instead of 21 narrow
 //    ones;
 //  * warps 2-17 (four per tensor-memory lane quadrant, 8 columns each) read a set after its
 //    MMAs completed, fold it into int64 sums and release it; after a task's last period
-//    (or every 64 periods) they write the contribution to C.
+//    (or every kFlushDrains periods) they write the contribution to C.
 // Warps 0 and 1 run their loops as whole warps (warp-uniform state and descriptors); one
 // elected lane issues each copy / tensor-core instruction.
 __global__ void __launch_bounds__(kRoleThreads, 1)
@@ -705,7 +700,7 @@ __global__ void __launch_bounds__(kRoleThreads, 1)
           asm volatile("tcgen05.fence::after_thread_sync;");
           const uint64_t soff = (uint64_t)((s * kStageBytes) >> 4);
           const uint32_t dbuf = tmem + (uint32_t)(buf * kAccCols);
-          // one elected lane issues the stage's 14 MMAs and its commits: the warp shares its
+          // one elected lane issues the stage's 12 MMAs and its commits: the warp shares its
           // scheduler with four busy drain warps, so the fewer instructions between two MMAs,
           // the less the tensor pipe waits for the next one
           if (elect_one()) {
@@ -715,7 +710,7 @@ __global__ void __launch_bounds__(kRoleThreads, 1)
 #pragma unroll
               for (int p = 1; p <= kS; ++p) {
                 const uint64_t adesc = sd0 + soff + (uint64_t)((ks * kAStep + (p - 1) * kTM * 32) >> 4);
-                // the first MMA of a period (p = 1, all 224 columns) overwrites the set
+                // the first MMA of a period (p = 1, all 192 columns) overwrites the set
                 const uint32_t acc = (first && ks == 0 && p == 1) ? 0u : 1u;
                 mma_bf16_issue(dbuf + (uint32_t)((p - 1) * kTN), adesc, bdesc, idesc_bf16(kTN * (kS + 1 - p)), acc);
               }

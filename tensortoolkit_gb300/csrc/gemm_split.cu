@@ -20,10 +20,10 @@
 //   two sets). Over 160 k the sums of levels 2..5 stay below 2^24 (level 5: 160 x 3 x 2^15) and
 //   are exact; level 6 may pass 2^24 by 1.1 and level 7 by 1.25 where every digit is at its
 //   limit, and then carry an FP32 rounding of one unit, 2^-48 or 2^-56. Every 160 k the drain
-//   warps read the levels and fold them into one int64 per output (units 2^-51); at the end of
-//   a task C (+)= sign 2^(ea + eb - 51) z, rounded to FP64 with integer operations.
-// D = 4000 matvec: k_gemm_split 122 / 97 -> 98 / 90 us (steps 0 / 3), k_pack_a 55 -> 48 us; error
-// against 64 bits 1.2e-13 -> 2.5e-14.
+//   warps read the levels and fold them into one int64 per output (units 2^-50); at the end of
+//   a task C (+)= sign 2^(ea + eb - 50) z, rounded to FP64 with integer operations.
+// D = 4000 matvec against the seven-slice form: k_gemm_split 122 / 97 -> 98 / 90 us (steps 0 / 3),
+// k_pack_a 55 -> 48 us; error against 64 bits 1.2e-13 -> 2.5e-14.
 //
 // Layout for the tensor cores: both operands K-major, no swizzle, in 8 x 16-byte core
 // matrices (leading-byte offset 128 B between the two core matrices of a 16-wide k step,
@@ -54,7 +54,7 @@ namespace {
 
 constexpr int kS = 6;                      // slices
 constexpr int kLevels = 6;                 // accumulators: levels 2..7
-constexpr int kUnit = 51;                  // the int64 sums are in units of 2^-kUnit
+constexpr int kUnit = 50;                  // the int64 sums are in units of 2^-kUnit
 constexpr int kTM = 128, kTN = 32, kTK = 64;
 constexpr int kATile = kTM * kTK * 2;      // bytes of one (row tile, k tile, slice): 16 KB
 constexpr int kBTile = kTN * kTK * 2;      // 4 KB
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(256) k_pack_a(const double* __restrict__ scr, 
     const int vrow = o.row_base + (int)row;
     const int vt = vrow / kTM, vr = vrow - vt * kTM;
     // tile layout [ks][slice][m_core][k_core][8 rows x 16 B]: the slices of a 16-wide k step
-    // are contiguous, so a 32-wide stage is one 48 KB copy
+    // are contiguous, so a stage is one 48 KB copy
     const int kt = k0 / kTK, ks = (k0 % kTK) >> 4;
     const int64_t tile = (int64_t)vt * o.ktiles + kt;
     uint8_t* dst = pack + o.pack_off + tile * (int64_t)(kS * kATile) + (int64_t)ks * (kS * 4096) + (vr >> 3) * 256 +
@@ -390,24 +390,29 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTM >> 4) << 24);
 }
 
-// Bounded waits spin for about 1 s of SM clock (2^31 cycles at the 2.07 GHz maximum),
-// checking the clock every 256 polls so the fast path is a bare try_wait.
+// Bounded waits last for about 1 s of SM clock (2^31 cycles at the 2.07 GHz maximum).
 constexpr long long kWaitCycles = 1ll << 31;
 
 // Operand pipeline: a stage holds one 32-wide k slab of all A slices (48 KB) and all B slices
 // (12 KB), each as it lies in the packed tile ([16-wide k step][slice][...]); 3 stages = 180 KB
 // of shared memory. Per 16-wide k step the A slices are 4 KB apart and the B slices form one
-// 192-row operand.
+// 192-row operand. (Seven 16-wide stages instead: 1260 cycles per 32 k against 1060; every stage
+// costs the tensor pipe a gap, and the producer is ahead with three.) Shared memory's bandwidth is
+// what the MMAs run against: per stage they read 90 KB of operands and the copies write 60 KB,
+// about 1200 cycles' worth, so the drain warps keep off it (their tile leaves by way of tensor
+// memory; staged through shared memory the D = 4000 matvec took 377 us instead of 358).
 constexpr int kStages = 3;
-constexpr int kKS = 32;                         // k per stage (2 MMA k-steps)
+constexpr int kKS = 32;                         // k per stage (2 MMA k steps)
 constexpr int kAStep = kS * kTM * 16 * 2;       // 24 KB: the A slices of one k step
 constexpr int kBStep = kS * kTN * 16 * 2;       // 6 KB: the B slices of one k step
 constexpr int kABytes = 2 * kAStep, kBBytes = 2 * kBStep;
 constexpr int kStageBytes = kABytes + kBBytes;  // 60 KB
 constexpr int kSmemBytes = kStages * kStageBytes + 1024;
 constexpr int kPeriod = kDrainK / kKS;          // stages between drains (5)
+// Sixteen drain warps of 8 columns rather than eight of 16: D = 4000 matvec 358 / 355 us, complex
+// Hubbard matvec (short tasks, several per tile) 394 / 424 us.
 constexpr int kDrainWarps = 16;                 // four per tensor-memory lane quadrant
-constexpr int kDrainCols = kTN / 4;             // columns per drain thread
+constexpr int kDrainCols = kTN / (kDrainWarps / 4);   // columns per drain thread
 constexpr int kRoleThreads = 64 + 32 * kDrainWarps;   // warp 0 producer, warp 1 MMA, warps 2-17 drain
 // Tensor memory: two accumulator sets, each 6 levels x 32 columns (level L at 32 (L - 2)).
 constexpr int kAccCols = kLevels * kTN;         // 192
@@ -416,7 +421,9 @@ constexpr int kSumCol = 2 * kAccCols;           // 384
 constexpr uint32_t kTmemAlloc = 512;
 static_assert(kDrainK % kKS == 0, "whole stages between drains");
 static_assert(kSumCol + 2 * kTN <= (int)kTmemAlloc, "tensor memory budget");
-constexpr int kFlushDrains = 12;                // the int64 sum of 12 x 160 k stays below 2^62
+constexpr int kFlushDrains = 24;                // the int64 sum of 24 x 160 k stays below 2^62
+constexpr float kMagic = 12582912.0f;           // 1.5 * 2^23: x + kMagic has the integer x in its low bits
+constexpr int kMagicBits = 0x4B400000;          // for |x| < 2^22
 
 __device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count));
@@ -425,7 +432,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t mbar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes));
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar));
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -438,12 +445,7 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(pred));
   return pred != 0;
 }
-// The tensor-core helpers below are called by a whole warp; the elected lane issues.
-__device__ __forceinline__ void tc_commit(uint32_t mbar) {
-  if (elect_one())
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar));
-}
-// The same, issued by the calling thread alone (the caller elects it).
+// Issued by the calling thread alone (the caller elects it).
 __device__ __forceinline__ void tc_commit_issue(uint32_t mbar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar));
 }
@@ -473,6 +475,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ldc(uint32_t taddr, uint32_t (&r)[kDrainCols]) {
+  if constexpr (kDrainCols == 16) tmem_ld16(taddr, r);
+  else tmem_ld8(taddr, r);
+}
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
@@ -485,15 +491,16 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
 __device__ __forceinline__ bool mbar_wait_or_abort(uint32_t mbar, uint32_t phase, const volatile int* abort_flag,
                                                    long long limit = kWaitCycles) {
   uint32_t done = 0;
-  const long long t0 = clock64();
-  while (true) {
-    for (int i = 0; i < 256; ++i) {
-      asm volatile(
-          "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-          : "=r"(done)
-          : "r"(mbar), "r"(phase));
-      if (done) return true;
-    }
+  long long t0 = 0;
+  for (bool first = true;; first = false) {
+    // suspends for up to 16 us at a time: a poll costs issue slots of the drain warps
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done)
+        : "r"(mbar), "r"(phase), "r"(16000u)
+        : "memory");
+    if (done) return true;
+    if (first) t0 = clock64();
     if (*abort_flag || clock64() - t0 > limit) return false;
   }
 }
@@ -506,12 +513,8 @@ __device__ __forceinline__ bool aborted(volatile int* abort_flag) {
 __device__ __forceinline__ bool wait_warp(uint32_t mbar, uint32_t phase, volatile int* abort_flag) {
   return __all_sync(0xffffffffu, mbar_wait_or_abort(mbar, phase, abort_flag));
 }
-// Bounded wait that ignores the abort flag: for the copies and tensor-core work a CTA issued
-// itself, which must land before it frees or leaves the memory they write.
-__device__ __forceinline__ bool wait_warp_own(uint32_t mbar, uint32_t phase) {
-  const int never = 0;
-  return __all_sync(0xffffffffu, mbar_wait_or_abort(mbar, phase, &never));
-}
+// (A wait for the copies and tensor-core work a CTA issued itself, which must land before it
+// frees or leaves the memory they write, passes a flag that is never set.)
 
 // The bounded wait itself, checked on the device: one warp waits on an mbarrier nothing
 // arrives on, with a limit of `limit` cycles, and reports 1 when the wait gave up (the
@@ -528,64 +531,142 @@ __global__ void __launch_bounds__(32) k_wait_selftest(long long limit, int* __re
   if (threadIdx.x == 0) *status = ok ? 0 : 1;
 }
 
-// Fold one drained accumulator set into the int64 sums z (units 2^-51) of this thread's row
-// and 8 columns. Level L holds integers times 2^(-8L), each below 2^24.4 over 160 k (see the
-// head of this file), so F2I gives them as they are; level 7 is rounded to units of 2^-51.
-// Level 2's units reach the high word only.
-__device__ __forceinline__ void drain_set(uint32_t lb, long long (&z)[kDrainCols]) {
-  // levels are read two at a time, one wait per pair
-  uint32_t r[kDrainCols], q[kDrainCols];
-  tmem_ld8(lb, r);                                       // level 2
-  tmem_ld8(lb + kTN, q);                                 // level 3
-  asm volatile("tcgen05.wait::ld.sync.aligned;");
-#pragma unroll
-  for (int c = 0; c < kDrainCols; ++c) {
-    const uint32_t h = (uint32_t)__float2int_rn(__uint_as_float(r[c]) * 0x1p19f);   // units 2^-19
-    z[c] += (long long)((uint64_t)h << 32);
-    z[c] += (long long)__float2int_rn(__uint_as_float(q[c]) * 0x1p24f) * (1ll << 27);
-  }
-  tmem_ld8(lb + 2 * kTN, r);                             // level 4
-  tmem_ld8(lb + 3 * kTN, q);                             // level 5
-  asm volatile("tcgen05.wait::ld.sync.aligned;");
-#pragma unroll
-  for (int c = 0; c < kDrainCols; ++c) {
-    z[c] += (long long)__float2int_rn(__uint_as_float(r[c]) * 0x1p32f) * (1ll << 19);
-    z[c] += (long long)__float2int_rn(__uint_as_float(q[c]) * 0x1p40f) * (1ll << 11);
-  }
-  tmem_ld8(lb + 4 * kTN, r);                             // level 6
-  tmem_ld8(lb + 5 * kTN, q);                             // level 7
-  asm volatile("tcgen05.wait::ld.sync.aligned;");
-#pragma unroll
-  for (int c = 0; c < kDrainCols; ++c)
-    z[c] += (long long)(__float2int_rn(__uint_as_float(r[c]) * 0x1p51f) + __float2int_rn(__uint_as_float(q[c]) * 0x1p51f));
+// a b + c in one instruction of the multiply-add pipe (shifts and adds of 64 bits are four, in the
+// busier pipe). b comes as a register, so that the product is not taken apart again.
+__device__ __forceinline__ uint64_t mad_wide(uint32_t a, uint32_t b, uint64_t c) {
+  uint64_t d;
+  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t mad_wide_s(int32_t a, int32_t b, uint64_t c) {
+  uint64_t d;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
 }
 
-// sum (+)= sign 2^(ea + eb - 51) z, each term rounded once to FP64; the tile's running sum
-// of this thread's 8 columns lives in tensor memory at tsum (16 columns). The first
-// contribution to a tile sets it, later ones add.
-__device__ __forceinline__ void fold_sums(const long long (&z)[kDrainCols], int ea, const int (&eb)[kDrainCols],
-                                          bool neg, uint32_t tsum, bool& written) {
-  uint32_t v[2 * kDrainCols];
-  if (written) {                                   // warp-uniform: later tasks of the tile add
-    tmem_ld16(tsum, v);
-    asm volatile("tcgen05.wait::ld.sync.aligned;");
+// What the kMagicBits of one drain add to a sum (modulo 2^64).
+constexpr uint64_t kDrainBias = (uint64_t)kMagicBits * ((1ull << 18) + (1ull << 10) + 1ull);
+
+// Fold one drained accumulator set into the int64 sums z (units 2^-50, plus kDrainBias) of this
+// thread's row and 8 columns. Level L holds integers times 2^(-8L). Levels 2 and 3 go through F2I
+// (level 2's units reach the high word only). For levels 4, 5 and 6 with 7 (rounded to units of
+// 2^-50) an addition of 1.5 2^23 leaves the integer in the low bits of the sum while it is below
+// 2^22, which the sum's exponent shows; where a warp has a larger one (up to 2^24.4: all digits of
+// a sign, near their limits) they go through F2I as well. F2I costs a warp eight cycles of a pipe
+// that nothing else here uses; the mix keeps that pipe and the two arithmetic ones about equally
+// busy (all six through F2I: 1500 cycles per drain of 16 warps, that pipe's rate; now 1150).
+__device__ __forceinline__ void drain_set(uint32_t lb, uint64_t (&z)[kDrainCols]) {
+  // levels are read two at a time, one wait per pair
+  uint32_t r[kDrainCols], q[kDrainCols], u[kDrainCols];
+  tmem_ldc(lb, r);                                       // level 2
+  tmem_ldc(lb + kTN, q);                                 // level 3
+  asm volatile("tcgen05.wait::ld.sync.aligned;");
+#pragma unroll
+  for (int c = 0; c < kDrainCols; ++c) {
+    const uint32_t h = (uint32_t)__float2int_rn(__uint_as_float(r[c]) * 0x1p18f);   // units 2^-18
+    z[c] += (uint64_t)h << 32;
+    z[c] = mad_wide_s(__float2int_rn(__uint_as_float(q[c]) * 0x1p24f), 1 << 26, z[c]);
+  }
+  tmem_ldc(lb + 2 * kTN, r);                             // level 4
+  tmem_ldc(lb + 3 * kTN, q);                             // level 5
+  asm volatile("tcgen05.wait::ld.sync.aligned;");
+  uint32_t off = 0;
+#pragma unroll
+  for (int c = 0; c < kDrainCols; ++c) {
+    u[c] = __float_as_uint(fmaf(__uint_as_float(r[c]), 0x1p32f, kMagic));
+    off |= u[c] ^ 0x4B000000u;
+  }
+  if (__any_sync(0xffffffffu, off & 0xFF800000u)) {
+#pragma unroll
+    for (int c = 0; c < kDrainCols; ++c)
+      u[c] = (uint32_t)(__float2int_rn(__uint_as_float(r[c]) * 0x1p32f) + kMagicBits);
+  }
+  off = 0;
+#pragma unroll
+  for (int c = 0; c < kDrainCols; ++c) {
+    z[c] = mad_wide(u[c], 1u << 18, z[c]);
+    u[c] = __float_as_uint(fmaf(__uint_as_float(q[c]), 0x1p40f, kMagic));
+    off |= u[c] ^ 0x4B000000u;
+  }
+  if (__any_sync(0xffffffffu, off & 0xFF800000u)) {
+#pragma unroll
+    for (int c = 0; c < kDrainCols; ++c)
+      u[c] = (uint32_t)(__float2int_rn(__uint_as_float(q[c]) * 0x1p40f) + kMagicBits);
+  }
+  tmem_ldc(lb + 4 * kTN, r);                             // level 6
+  tmem_ldc(lb + 5 * kTN, q);                             // level 7
+#pragma unroll
+  for (int c = 0; c < kDrainCols; ++c) z[c] = mad_wide(u[c], 1u << 10, z[c]);
+  asm volatile("tcgen05.wait::ld.sync.aligned;");
+  off = 0;
+#pragma unroll
+  for (int c = 0; c < kDrainCols; ++c) {
+    u[c] = __float_as_uint(fmaf(__uint_as_float(r[c]), 0x1p50f, fmaf(__uint_as_float(q[c]), 0x1p50f, kMagic)));
+    off |= u[c] ^ 0x4B000000u;
+  }
+  if (__any_sync(0xffffffffu, off & 0xFF800000u)) {
+#pragma unroll
+    for (int c = 0; c < kDrainCols; ++c)
+      u[c] = (uint32_t)(__float2int_rn(__uint_as_float(r[c]) * 0x1p50f) +
+                        __float2int_rn(__uint_as_float(q[c]) * 0x1p50f) + kMagicBits);
+  }
+#pragma unroll
+  for (int c = 0; c < kDrainCols; ++c) z[c] = mad_wide(u[c], 1u, z[c]);
+}
+
+// x = sign 2^(ea + eb - 50) z, each rounded once to FP64, plus the tile's running sum of this
+// thread's 8 columns where there is one (in tensor memory at tsum, 16 columns). Lane c (mod 8)
+// holds column c's eb.
+// Where no result can be subnormal or infinite (scales between 2^-450 and 2^450) and every |z| is
+// zero or has a bit in its high word, a product with 2^(lz - 1), which adds half an ulp at once,
+// puts the leading one at bit 62 (|z| < 2^62; a tie, which takes more than 53 bits, goes away from
+// zero): a third of the general form's instructions. Zeros are common: padding, and rows or
+// columns without data.
+__device__ __forceinline__ void fold_sums(const uint64_t (&z)[kDrainCols], int ea, int eb, bool neg, uint32_t tsum,
+                                          bool add, double (&x)[kDrainCols]) {
+  uint32_t low_only = 0;
+  uint64_t a[kDrainCols];
+#pragma unroll
+  for (int c = 0; c < kDrainCols; ++c) {
+    const uint32_t sg = (uint32_t)((int32_t)(z[c] >> 32) >> 31);
+    a[c] = (z[c] ^ (((uint64_t)sg << 32) | sg)) + (sg & 1u);
+    if ((uint32_t)(a[c] >> 32) == 0) low_only |= (uint32_t)a[c];
+  }
+  if (__all_sync(0xffffffffu, low_only == 0 && abs(ea) <= 450 && abs(eb) <= 450)) {
+    // (biased exponent - 1) of a value whose high word has its leading one at bit m: 1054 + m + e
+    const uint32_t ka = (uint32_t)(1054 + ea - kUnit) << 20;
+    const uint32_t kb = (uint32_t)eb << 20;
 #pragma unroll
     for (int c = 0; c < kDrainCols; ++c) {
-      const double x = scaled_i64(z[c], ea + eb[c] - kUnit, neg) + __hiloint2double((int)v[2 * c + 1], (int)v[2 * c]);
-      v[2 * c] = (uint32_t)__double2loint(x);
-      v[2 * c + 1] = (uint32_t)__double2hiint(x);
+      const uint32_t ah = (uint32_t)(a[c] >> 32);
+      uint32_t m, pow;
+      asm("bfind.u32 %0, %1;" : "=r"(m) : "r"(ah));                                // 0xFFFFFFFF for zero
+      asm("shr.u32 %0, %1, %2;" : "=r"(pow) : "r"(0x40000000u), "r"(m));           // 0 for zero
+      const uint64_t lo = mad_wide((uint32_t)a[c], pow, 0x200u);
+      const uint32_t mh = ah * pow + (uint32_t)(lo >> 32);
+      const uint32_t hi = (mh >> 10) + __shfl_sync(0xffffffffu, kb, c) + (m * (1u << 20) + ka);
+      x[c] = __hiloint2double((int)((ah ? hi : 0u) | ((uint32_t)(z[c] >> 32) & 0x80000000u)),
+                              (int)__funnelshift_r((uint32_t)lo, mh, 10));
     }
   } else {
 #pragma unroll
-    for (int c = 0; c < kDrainCols; ++c) {
-      const double x = scaled_i64(z[c], ea + eb[c] - kUnit, neg);
-      v[2 * c] = (uint32_t)__double2loint(x);
-      v[2 * c + 1] = (uint32_t)__double2hiint(x);
+    for (int c = 0; c < kDrainCols; ++c)
+      x[c] = scaled_i64((long long)z[c], ea + __shfl_sync(0xffffffffu, eb, c) - kUnit, false);
+  }
+  if (neg) {
+#pragma unroll
+    for (int c = 0; c < kDrainCols; ++c) {          // zero stays +0, as in the general form
+      const long long b = __double_as_longlong(x[c]);
+      x[c] = __longlong_as_double(b ? b ^ (long long)0x8000000000000000ull : 0ll);
     }
   }
-  tmem_st16(tsum, v);
-  asm volatile("tcgen05.wait::st.sync.aligned;");
-  written = true;
+  if (add) {                                       // warp-uniform: later tasks of the tile
+    uint32_t v[2 * kDrainCols];
+    for (int h = 0; h < kDrainCols / 8; ++h) tmem_ld16(tsum + 16 * h, v + 16 * h);
+    asm volatile("tcgen05.wait::ld.sync.aligned;");
+#pragma unroll
+    for (int c = 0; c < kDrainCols; ++c) x[c] += __hiloint2double((int)v[2 * c + 1], (int)v[2 * c]);
+  }
 }
 
 // Warp-specialised split GEMM. All roles walk the same static sequence of work items
@@ -603,8 +684,10 @@ __device__ __forceinline__ void fold_sums(const long long (&z)[kDrainCols], int 
 //  * warps 2-17 (four per tensor-memory lane quadrant, 8 columns each) read a set after its
 //    MMAs completed, fold it into int64 sums and release it; after a task's last period
 //    (or every kFlushDrains periods) they write the contribution to C.
-// Warps 0 and 1 run their loops as whole warps (warp-uniform state and descriptors); one
-// elected lane issues each copy / tensor-core instruction.
+// Warps 0 and 1 run their loops in one elected lane.
+// D = 4000 matvec, steps 0 / 3: 98 / 90 -> 86 / 76 us against whole-warp loops, records and scales
+// loaded by each task for itself, F2I for every level and the general form of the FP64 rounding.
+// The MMAs alone take about 65 us (99 stages of 1200 cycles).
 __global__ void __launch_bounds__(kRoleThreads, 1)
     k_gemm_split(const SplitWork* __restrict__ items, const int32_t* __restrict__ item_off,
                  const uint8_t* __restrict__ apack, const uint8_t* __restrict__ bpack,
@@ -641,135 +724,165 @@ __global__ void __launch_bounds__(kRoleThreads, 1)
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    uint32_t g = 0;
-    SplitWork nx;
-    if (beg < end) nx = items[beg];
-    for (int it = beg; it < end && !aborted(&s_abort); ++it) {
-      const SplitWork w = nx;
-      if (it + 1 < end) nx = items[it + 1];            // prefetch the next step
-      const int nst = (w.k + kKS - 1) / kKS;
+    if (elect_one()) {
+      uint32_t g = 0;      // stages filled
+      int st = 0;          // g % kStages
+      uint32_t ph = 1;     // parity of the stage's last release (the first round waits for none)
+      SplitWork nx;
+      if (beg < end) nx = items[beg];
       bool ok = true;
-      for (int j = 0; j < nst; ++j, ++g) {
-        const int s = g % kStages;
-        if (g >= (uint32_t)kStages && !wait_warp(smem_u32(&empty_bar[s]), ((g / kStages) - 1) & 1, &s_abort)) {
-          if (lane == 0) fail();
-          ok = false;
-          break;
-        }
-        const int kt = j >> 1, half = j & 1;
-        const uint8_t* ga = apack + w.a_pack + ((int64_t)w.tm * w.ktiles + kt) * (kS * kATile) + half * kABytes;
-        const uint8_t* gb = bpack + w.b_pack + ((int64_t)w.tn * w.ktiles + kt) * (kS * kBTile) + half * kBBytes;
-        const uint32_t sa = sbase + s * kStageBytes;
-        const uint32_t fb = smem_u32(&full_bar[s]);
-        if (elect_one()) {
-          mbar_expect_tx(fb, kStageBytes);
-          bulk_g2s(sa, ga, kABytes, fb);
-          bulk_g2s(sa + kABytes, gb, kBBytes, fb);
-        }
-        __syncwarp();
-      }
-      if (!ok) break;
-    }
-    // copies still in flight are waited for by the MMA warp (every issued stage is consumed
-    // on the normal path); on abort wait for the tail of issued stages here
-    if (aborted(&s_abort)) {
-      for (uint32_t x = (g > (uint32_t)kStages ? g - kStages : 0); x < g; ++x)
-        wait_warp_own(smem_u32(&full_bar[x % kStages]), (x / kStages) & 1);
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ tensor-core issuer
-    // descriptor of stage 0 at byte 0; every operand is a fixed byte offset from it
-    const uint64_t sd0 = smem_desc(sbase);
-    uint32_t g = 0, d = 0;
-    bool ok = true;
-    int nst_next = beg < end ? items[beg].k : 0;
-    for (int it = beg; it < end && ok && !aborted(&s_abort); ++it) {
-      const int nst = (nst_next + kKS - 1) / kKS;
-      if (it + 1 < end) nst_next = items[it + 1].k;   // prefetch the next step
-      {
+      for (int it = beg; it < end && ok; ++it) {
+        const SplitWork w = nx;
+        if (it + 1 < end) nx = items[it + 1];            // prefetch the next step
+        const int nst = (w.k + kKS - 1) / kKS;
+        // a row tile's k steps lie end to end (two stages to a 64-wide k tile)
+        const uint8_t* ga = apack + w.a_pack + (int64_t)w.tm * w.ktiles * (kS * kATile);
+        const uint8_t* gb = bpack + w.b_pack + (int64_t)w.tn * w.ktiles * (kS * kBTile);
         for (int j = 0; j < nst; ++j, ++g) {
-          const int s = g % kStages;
-          const int buf = d & 1;
-          const bool first = (j % kPeriod) == 0;
-          const bool drain = (j % kPeriod) == kPeriod - 1 || j + 1 == nst;
-          if (first && d >= 2 && !wait_warp(smem_u32(&acce_bar[buf]), ((d / 2) - 1) & 1, &s_abort)) {
+          if (g >= (uint32_t)kStages && !mbar_wait_or_abort(smem_u32(&empty_bar[st]), ph, &s_abort)) {
             ok = false;
             break;
           }
-          if (!wait_warp(smem_u32(&full_bar[s]), (g / kStages) & 1, &s_abort)) { ok = false; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          const uint64_t soff = (uint64_t)((s * kStageBytes) >> 4);
-          const uint32_t dbuf = tmem + (uint32_t)(buf * kAccCols);
-          // one elected lane issues the stage's 12 MMAs and its commits: the warp shares its
-          // scheduler with four busy drain warps, so the fewer instructions between two MMAs,
-          // the less the tensor pipe waits for the next one
-          if (elect_one()) {
-#pragma unroll
-            for (int ks = 0; ks < kKS / 16; ++ks) {
-              const uint64_t bdesc = sd0 + soff + (uint64_t)((kABytes + ks * kBStep) >> 4);
-#pragma unroll
-              for (int p = 1; p <= kS; ++p) {
-                const uint64_t adesc = sd0 + soff + (uint64_t)((ks * kAStep + (p - 1) * kTM * 32) >> 4);
-                // the first MMA of a period (p = 1, all 192 columns) overwrites the set
-                const uint32_t acc = (first && ks == 0 && p == 1) ? 0u : 1u;
-                mma_bf16_issue(dbuf + (uint32_t)((p - 1) * kTN), adesc, bdesc, idesc_bf16(kTN * (kS + 1 - p)), acc);
-              }
-            }
-            tc_commit_issue(smem_u32(&empty_bar[s]));
-            if (drain) tc_commit_issue(smem_u32(&accf_bar[buf]));
+          const uint32_t sa = sbase + st * kStageBytes;
+          const uint32_t fb = smem_u32(&full_bar[st]);
+          mbar_expect_tx(fb, kStageBytes);
+          bulk_g2s(sa, ga, kABytes, fb);
+          bulk_g2s(sa + kABytes, gb, kBBytes, fb);
+          ga += kABytes;
+          gb += kBBytes;
+          if (++st == kStages) {
+            st = 0;
+            ph ^= 1;
           }
-          __syncwarp();
-          if (drain) ++d;
         }
+        if (ok && s_abort) ok = false;
+      }
+      // copies still in flight are waited for by the MMA warp (every issued stage is consumed on
+      // the normal path); on abort wait for the tail of issued stages here
+      if (!ok) {
+        fail();
+        const int never = 0;
+        for (uint32_t x = (g > (uint32_t)kStages ? g - kStages : 0); x < g; ++x)
+          mbar_wait_or_abort(smem_u32(&full_bar[x % kStages]), (x / kStages) & 1, &never);
       }
     }
-    if (!ok && lane == 0) fail();
-    // all tensor-core work issued by this warp completes before the memory is released
-    tc_commit(smem_u32(&fin_bar));
-    wait_warp_own(smem_u32(&fin_bar), 0);
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ tensor-core issuer
+    // one lane walks the stages: the warp shares its scheduler with four busy drain warps, so
+    // the fewer instructions between two stages' MMAs, the less the tensor pipe waits
+    if (elect_one()) {
+      // descriptor of stage 0 at byte 0; every operand is a fixed byte offset from it
+      const uint64_t sd0 = smem_desc(sbase);
+      int st = 0;
+      uint32_t ph = 0, d = 0;
+      bool ok = true;
+      int k_next = beg < end ? items[beg].k : 0;
+      for (int it = beg; it < end && ok; ++it) {
+        const int nst = (k_next + kKS - 1) / kKS;
+        if (it + 1 < end) k_next = items[it + 1].k;   // prefetch the next step
+        int left = 0;                                 // stages left of the period
+        for (int j = 0; j < nst; ++j) {
+          const int buf = d & 1;
+          const bool first = left == 0;
+          if (first) {
+            left = min(kPeriod, nst - j);
+            if (d >= 2 && !mbar_wait_or_abort(smem_u32(&acce_bar[buf]), ((d / 2) - 1) & 1, &s_abort)) {
+              ok = false;
+              break;
+            }
+          }
+          if (!mbar_wait_or_abort(smem_u32(&full_bar[st]), ph, &s_abort)) {
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          const uint64_t adesc = sd0 + (uint64_t)((st * kStageBytes) >> 4);
+          const uint64_t bdesc = adesc + (uint64_t)(kABytes >> 4);
+          const uint32_t dbuf = tmem + (uint32_t)(buf * kAccCols);
+#pragma unroll
+          for (int ks = 0; ks < kKS / 16; ++ks) {
+#pragma unroll
+            for (int p = 1; p <= kS; ++p) {
+              // the first MMA of a period (p = 1, all 192 columns) overwrites the set
+              const uint32_t acc = (first && ks == 0 && p == 1) ? 0u : 1u;
+              mma_bf16_issue(dbuf + (uint32_t)((p - 1) * kTN),
+                             adesc + (uint64_t)((ks * kAStep + (p - 1) * kTM * 32) >> 4),
+                             bdesc + (uint64_t)((ks * kBStep) >> 4), idesc_bf16(kTN * (kS + 1 - p)), acc);
+            }
+          }
+          tc_commit_issue(smem_u32(&empty_bar[st]));
+          if (--left == 0) {
+            tc_commit_issue(smem_u32(&accf_bar[buf]));
+            ++d;
+          }
+          if (++st == kStages) {
+            st = 0;
+            ph ^= 1;
+          }
+        }
+        if (ok && s_abort) ok = false;
+      }
+      if (!ok) fail();
+      // all tensor-core work issued here completes before the memory is released
+      tc_commit_issue(smem_u32(&fin_bar));
+      const int never = 0;
+      mbar_wait_or_abort(smem_u32(&fin_bar), 0, &never);
+    }
+    __syncwarp();
   } else if (warp >= 2) {
     // ------------------------------------------------------------ drain / epilogue
     const int quad = warp & 3;                       // tensor-memory lanes 32 * quad .. + 31
     const int cpart = (warp - 2) >> 2;               // columns 8 * cpart .. + 7 of the tile
     const int row_in_tile = quad * 32 + lane;
+    const int cl = cpart * kDrainCols + (lane & (kDrainCols - 1));   // this lane's column of the tile
     uint32_t d = 0;
     bool stop = false, written = false;
     // outputs of the tile that a non-finite operand row or column reaches (bit c: column c);
     // they are stored as NaN (FP64 gives NaN or an infinity there; the slices cannot carry it)
     uint32_t poison = 0;
     const uint32_t tsum = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(kSumCol + 2 * cpart * kDrainCols);
+    // the next task's record, scale fields (of this lane's row and column) and place of the row
+    // in C are fetched one task ahead: two dependent loads, ~2000 cycles where a task's drain,
+    // fold and store take 3000-5000
+    SplitWork nx{};
+    int nfa = 0, nfb = 0;
+    long long nrow = -1;
+    auto fetch = [&]() {
+      const int row = nx.tm * kTM + row_in_tile;
+      nfa = row < nx.m ? aexp[nx.a_exp + row] : 0;
+      nfb = nx.tn * kTN + cl < nx.n ? bexp[nx.b_exp + nx.tn * kTN + cl] : 0;
+      nrow = (nx.flags & 2) && row < nx.m ? __ldg(row_map + nx.row_map + row) : -1ll;
+    };
+    if (beg < end) {
+      nx = items[beg];
+      fetch();
+    }
     for (int it = beg; it < end && !stop && !aborted(&s_abort); ++it) {
-      const SplitWork w = items[it];
-      const int row = w.tm * kTM + row_in_tile;
-      const int col0 = w.tn * kTN + cpart * kDrainCols;
-      const int nst = (w.k + kKS - 1) / kKS;
-      if (w.flags & 1) {
+      const int k = nx.k, n = nx.n, flags = nx.flags;
+      const bool neg = nx.sign < 0;
+      const int tcol = nx.tn * kTN;
+      const int fa = nfa, fb = nfb;
+      const long long rmap = nrow;
+      bool fetched = it + 1 >= end;
+      if (!fetched) nx = items[it + 1];
+      const int nst = (k + kKS - 1) / kKS;
+      if (flags & 1) {
         written = false;
         poison = 0;
       }
-      // this row's place in C, fetched early for the tile's store
-      const long long rmap = (w.flags & 2) && row < w.m ? __ldg(row_map + w.row_map + row) : -1ll;
-      // scale exponents, fetched while the first period is still on the tensor cores
-      const int fa = row < w.m ? aexp[w.a_exp + row] : 0;
-      const int ea = exp_of_field(fa);
+      poison |= __ballot_sync(0xffffffffu, fb == 2047) & ((1u << kDrainCols) - 1);
       if (fa == 2047) poison = (1u << kDrainCols) - 1;
-      int eb[kDrainCols];
-#pragma unroll
-      for (int c = 0; c < kDrainCols; ++c) {
-        const int fb = col0 + c < w.n ? bexp[w.b_exp + col0 + c] : 0;
-        eb[c] = exp_of_field(fb);
-        if (fb == 2047) poison |= 1u << c;
-      }
-      long long z[kDrainCols];
+      const int ea = exp_of_field(fa), eb = exp_of_field(fb);
+      uint64_t z[kDrainCols];
       // the task's periods in chunks of kFlushDrains, each folded on its own, so the int64
       // sums stay in range for any k
       for (int j0 = 0; j0 < nst && !stop; j0 += kFlushDrains * kPeriod) {
         const int j1 = min(nst, j0 + kFlushDrains * kPeriod);
+        const uint64_t z0 = 0ull - (uint64_t)((j1 - j0 + kPeriod - 1) / kPeriod) * kDrainBias;
 #pragma unroll
-        for (int c = 0; c < kDrainCols; ++c) z[c] = 0;
-        for (int j = j0; j < j1; ++j) {
-          const bool drain = (j % kPeriod) == kPeriod - 1 || j + 1 == nst;
-          if (!drain) continue;
+        for (int c = 0; c < kDrainCols; ++c) z[c] = z0;
+        for (int j = j0; j < j1; j += kPeriod) {
           const int buf = d & 1;
           if (!wait_warp(smem_u32(&accf_bar[buf]), (d / 2) & 1, &s_abort)) {
             if (lane == 0) fail();
@@ -782,44 +895,69 @@ __global__ void __launch_bounds__(kRoleThreads, 1)
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&acce_bar[buf]));
           ++d;
+          if (!fetched) {
+            fetch();
+            fetched = true;
+          }
         }
         if (stop) break;
-        fold_sums(z, ea, eb, w.sign < 0, tsum, written);
-      }
-      // one store per tile after its last task (a C tile belongs to exactly one CTA). The sums
-      // are read back in the 16 x 256-bit shape, so that four consecutive lanes hold four
-      // consecutive columns of one row and each store instruction writes 32-byte pieces of 8
-      // rows (a lane-per-row store would write 32 separate 8-byte pieces). Row places and
-      // non-finite masks come from the lane that owns the row.
-      if (!stop && (w.flags & 2)) {
-        uint32_t v[4 * kDrainCols];
-        const uint32_t tb = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(kSumCol + 2 * cpart * kDrainCols);
-        tmem_ld_16x256b(tb, v);
-        tmem_ld_16x256b(tb + 8u, v + 4);
-        tmem_ld_16x256b(tb + (16u << 16), v + 8);
-        tmem_ld_16x256b(tb + (16u << 16) + 8u, v + 12);
-        asm volatile("tcgen05.wait::ld.sync.aligned;");
-        const int cq = lane & 3, rq = lane >> 2;
+        double x[kDrainCols];
+        fold_sums(z, ea, eb, neg, tsum, written, x);
+        if (j1 < nst || !(flags & 2)) {              // more to come: the sum stays in tensor memory
+          uint32_t v[2 * kDrainCols];
 #pragma unroll
-        for (int lh = 0; lh < 2; ++lh)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int rl = 16 * lh + 8 * h + rq;       // the row's lane in this warp
-            const long long rm = __shfl_sync(0xffffffffu, rmap, rl);
-            const uint32_t pz = __shfl_sync(0xffffffffu, poison, rl);
-            if (rm >= 0) {
-#pragma unroll
-              for (int ch = 0; ch < 2; ++ch) {
-                const int c = 4 * ch + cq;
-                if (col0 + c < w.n) {
-                  const uint32_t* x = v + 8 * lh + 4 * ch + 2 * h;
-                  C[rm + col0 + c] = (pz >> c) & 1u ? __longlong_as_double(0x7FF8000000000000ll)
-                                                    : __hiloint2double((int)x[1], (int)x[0]);
-                }
-              }
-            }
+          for (int c = 0; c < kDrainCols; ++c) {
+            v[2 * c] = (uint32_t)__double2loint(x[c]);
+            v[2 * c + 1] = (uint32_t)__double2hiint(x[c]);
           }
+          for (int h = 0; h < kDrainCols / 8; ++h) tmem_st16(tsum + 16 * h, v + 16 * h);
+          asm volatile("tcgen05.wait::st.sync.aligned;");
+          written = true;
+          continue;
+        }
+        // one store per tile (a C tile belongs to exactly one CTA). The sums go through tensor
+        // memory and are read back in the 16 x 256-bit shape, so that four consecutive lanes hold
+        // four consecutive columns of one row and each store instruction writes 32-byte pieces of
+        // 8 rows (a lane-per-row store would write 32 separate 8-byte pieces; whole rows by way of
+        // shared memory take from the bandwidth that the tensor cores read their operands with).
+        // Row places come from the lane that owns the row.
+        if (__any_sync(0xffffffffu, poison)) {
+#pragma unroll
+          for (int c = 0; c < kDrainCols; ++c)
+            if ((poison >> c) & 1u) x[c] = __longlong_as_double(0x7FF8000000000000ll);
+        }
+        uint32_t v[2 * kDrainCols];
+#pragma unroll
+        for (int c = 0; c < kDrainCols; ++c) {
+          v[2 * c] = (uint32_t)__double2loint(x[c]);
+          v[2 * c + 1] = (uint32_t)__double2hiint(x[c]);
+        }
+#pragma unroll
+        for (int h = 0; h < kDrainCols / 8; ++h) tmem_st16(tsum + 16 * h, v + 16 * h);
+        const uint64_t addr = rmap >= 0 ? reinterpret_cast<uint64_t>(C + (rmap + tcol + cpart * kDrainCols)) : 0ull;
+        asm volatile("tcgen05.wait::st.sync.aligned;");
+#pragma unroll
+        for (int h = 0; h < kDrainCols / 4; ++h) {          // four columns at a time
+          tmem_ld_16x256b(tsum + 8u * h, v + 8 * h);
+          tmem_ld_16x256b(tsum + (16u << 16) + 8u * h, v + 8 * h + 4);
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;");
+        const int cq = lane & 3, left = n - tcol - cpart * kDrainCols - cq;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {                       // rows 8 r + lane / 4 of the warp's 32
+          const uint64_t ra = __shfl_sync(0xffffffffu, addr, 8 * r + (lane >> 2));
+#pragma unroll
+          for (int h = 0; h < kDrainCols / 4; ++h) {
+            const uint32_t* y = v + 8 * h + 2 * r;
+            // predicated, not branched around
+            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u64 p, %0, 0;\n\t@p st.global.f64 [%1], %2;\n\t}" ::"l"(
+                             4 * h < left ? ra : 0ull),
+                         "l"(ra + 8u * (uint32_t)(4 * h + cq)), "d"(__hiloint2double((int)y[1], (int)y[0]))
+                         : "memory");
+          }
+        }
       }
+      if (!fetched && !stop) fetch();
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -1043,7 +1181,7 @@ void SplitPlan::build(const CtrctPlan& p, cudaStream_t s) {
   std::vector<int64_t> cost(nstacks, 0);
   for (int32_t si = 0; si < nstacks; ++si) {
     const GemmCBlk& c0 = g.cblk[stack_cblk0[si]];
-    for (int32_t t = c0.t0; t < c0.t1; ++t) cost[si] += 2 * ((cw * g.task[t].k + 31) / 32) + 1;
+    for (int32_t t = c0.t0; t < c0.t1; ++t) cost[si] += 2 * ((cw * g.task[t].k + kKS - 1) / kKS) + 1;
   }
   std::stable_sort(tiles.begin(), tiles.end(), [&](const GemmTile& x, const GemmTile& y) { return cost[x.cblk] > cost[y.cblk]; });
   grid = (int)std::min<int64_t>((int64_t)tiles.size(), std::max(1, p.ctx->num_sms));

@@ -174,7 +174,7 @@ struct SplitPlan {
   std::vector<int32_t> work_off;  // grid + 1 offsets into work
   int grid = 0;
   std::vector<int2> b_col_tiles;  // (B operand, 32-column tile) items of the B packing kernel
-  int row_exp_grid = 1, pack_a_grid = 1, pack_b_grid = 1;   // one wave of resident CTAs of each
+  int row_exp_grid = 1, pack_a_grid = 1, pack_b_grid = 1;   // one wave of resident CTAs, four for the packs
   int64_t n_a_chunks = 0, n_a_pchunks = 0, n_a_rows = 0;
   bool row_warp = false;          // A row scales one warp per row (long rows) or by chunks
   bool a_fields_external = false; // A row scales written by the kernel producing A (matvec)

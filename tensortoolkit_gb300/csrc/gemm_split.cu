@@ -232,6 +232,11 @@ __global__ void __launch_bounds__(256) k_row_field_rows(const double* __restrict
 // 16-byte chunks, 8 consecutive k each), numbered per operand in (128-row tile, k step, row)
 // order, so consecutive threads take consecutive rows and their 16-byte plane words land
 // side by side. CTA b takes the contiguous range [b per, (b + 1) per) of all operands' items.
+// Every lane reads its own row: the cache takes a line per lane and load, so pairs are loaded at
+// once where the row's address allows it. Bound by that and by memory latency. D = 4000 (10.0 M
+// elements): 47 -> 43 us, complex Hubbard 38 -> 26 us with the pair loads and four waves of CTAs
+// (reading the rows together and handing them out by shuffles or through shared memory: 50 and
+// 60 us).
 __global__ void __launch_bounds__(256) k_pack_a(const double* __restrict__ scr, const double* __restrict__ src,
                                                 const SplitOperand* __restrict__ ops, int nops, int64_t total,
                                                 const int32_t* __restrict__ exps, uint8_t* __restrict__ pack) {
@@ -266,6 +271,7 @@ __global__ void __launch_bounds__(256) k_pack_a(const double* __restrict__ scr, 
     // tile layout [ks][slice][m_core][k_core][8 rows x 16 B]: the slices of a 16-wide k step
     // are contiguous, so a stage is one 48 KB copy
     const int kt = k0 / kTK, ks = (k0 % kTK) >> 4;
+    const bool aligned = !(reinterpret_cast<uintptr_t>(src_row) & 15);
     const int64_t tile = (int64_t)vt * o.ktiles + kt;
     uint8_t* dst = pack + o.pack_off + tile * (int64_t)(kS * kATile) + (int64_t)ks * (kS * 4096) + (vr >> 3) * 256 +
                    (vr & 7) * 16;
@@ -275,8 +281,20 @@ __global__ void __launch_bounds__(256) k_pack_a(const double* __restrict__ scr, 
       if (kb >= o.cols) break;
       uint64_t y[8];
       uint32_t sg[8];
+      double x[8];
+      if (aligned && kb + 8 <= o.cols) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) y[j] = digits_of((kb + j < o.cols) ? __ldg(src_row + kb + j) : 0.0, e, sg[j]);
+        for (int j = 0; j < 8; j += 2) {
+          const double2 v = __ldg(reinterpret_cast<const double2*>(src_row + kb + j));
+          x[j] = v.x;
+          x[j + 1] = v.y;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = kb + j < o.cols ? __ldg(src_row + kb + j) : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) y[j] = digits_of(x[j], e, sg[j]);
       store_planes(y, sg, dst + half * 128, 4096);
     }
   }
@@ -1263,13 +1281,15 @@ void SplitPlan::build(const CtrctPlan& p, cudaStream_t s) {
                                                                  (int64_t)std::max(1, per_sm) * p.ctx->num_sms));
     }
     QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pack_a, 256, 0));
+    // four waves: CTAs of one wave finish up to a quarter apart (their ranges differ in locality).
+    // k_pack_a: see there; k_pack_b_cols, complex Hubbard: 27 -> 23.5 us
     pack_a_grid = (int)std::max<int64_t>(1, std::min<int64_t>((n_a_pchunks + 255) / 256,
-                                                              (int64_t)std::max(1, per_sm) * p.ctx->num_sms));
+                                                              (int64_t)std::max(1, per_sm) * p.ctx->num_sms * 4));
     if (p.a.dtype == QLTG_C128)
       QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pack_b_cols<true>, 256, 0));
     else
       QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pack_b_cols<false>, 256, 0));
-    pack_b_grid = std::max(1, std::min((int)b_col_tiles.size(), std::max(1, per_sm) * p.ctx->num_sms));
+    pack_b_grid = std::max(1, std::min((int)b_col_tiles.size(), std::max(1, per_sm) * p.ctx->num_sms * 4));
   }
   d_a_ops = upload(a_ops, s);
   d_b_ops = upload(b_ops, s);

@@ -344,7 +344,7 @@ void launch_f64(const GemmSchedule& g, const Operands& op, void* c, int num_sms,
   }
 }
 
-// CTAs of one full wave: the grid-stride loop then has no partial second wave.
+// CTAs of one full wave.
 template <typename T>
 int skinny_wave(int num_sms) {
   static int per_sm = [] {
@@ -356,7 +356,11 @@ int skinny_wave(int num_sms) {
 }
 
 int skinny_grid(int items, bool cplx, int num_sms) {
-  const int wave = cplx ? skinny_wave<double2>(num_sms) : skinny_wave<double>(num_sms);
+  // Complex: up to four waves. An equal share of passes per warp is not an equal share of work
+  // (their entries differ), and with one wave the SMs finish up to a sixth apart: Hubbard MPO steps
+  // 71 / 75 -> 62 / 69 us. The real passes are four times shorter and the start of a CTA weighs
+  // more: D = 4000 MPO 120 us with one wave, 122 with four.
+  const int wave = cplx ? 4 * skinny_wave<double2>(num_sms) : skinny_wave<double>(num_sms);
   const int per_cta = kSkinnyThreads / 32;
   return std::max(1, std::min((items + per_cta - 1) / per_cta, wave));
 }

@@ -40,3 +40,19 @@ def test_qr_block_shapes(gpu, dtype, tall):
             assert np.all(np.diagonal(rr).imag == 0)
         assert rel_frob(q.block(b), rq) <= 1e-11, shape
         assert rel_frob(r.block(b), rr) <= 1e-11, shape
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.complex128])
+def test_qr_panel_beside_update(gpu, dtype):
+    """Enough work that the first updates are cut in two, the next panel running beside the second
+    part (at least two 128-row items per SM), then not any more; some blocks have no second part,
+    some no next panel. Tall blocks are well conditioned (below 20), the wide ones' leading squares
+    at most 1e4: the bound above holds."""
+    shapes = [(800, 640), (96, 640), (700, 500), (33, 600), (900, 420), (640, 96), (300, 65), (64, 64), (31, 40)]
+    t = _blocks(shapes, dtype, 12)
+    q, r = QR(DTensor.from_host(t), 1, [0])
+    q, r = q.to_host(), r.to_host()
+    for b, shape in enumerate(shapes):
+        rq, rr = np.linalg.qr(t.block(b))
+        assert rel_frob(q.block(b), rq) <= 1e-11, shape
+        assert rel_frob(r.block(b), rr) <= 1e-11, shape

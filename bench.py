@@ -151,11 +151,11 @@ class ClockSampler:
 
 # DRAM bytes (read + write) per launch of the dominant kernel, from one ncu capture of
 # `python bench.py --profile --profile-case step0|step3` (split) and `--profile --mode fp64`
-# (summaries: profiles/k_gemm_split_d4000.txt, profiles/k_gemm_dfma_d4000.txt). Keyed by
+# (summaries: profiles/k_gemm_split_d4000.txt, profiles/k_gemm_f64_d4000.txt). Keyed by
 # matvec step.
 NCU_TRAFFIC = {
-    "split": {0: 117.4e6, 3: 228.9e6},
-    "fp64": {0: 84.6e6, 3: 167.7e6},
+    "split": {0: 104.5e6, 3: 202.6e6},
+    "fp64": {0: 78.9e6, 3: 132.7e6},
 }
 
 

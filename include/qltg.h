@@ -169,7 +169,7 @@ QLTG_API int qltg_ctrct_plan_set_schedule(qltg_ctrct_plan* plan, int32_t f64_til
  * the slowest candidate (ms[2 mode], ms[2 mode + 1]). Any out-pointer may be NULL. */
 QLTG_API int qltg_ctrct_plan_get_schedule(const qltg_ctrct_plan* plan, int32_t* f64_tile_rows, int32_t* split_stack,
                                           int32_t* tuned, float* ms);
-/* Autotune the schedule of `mode`: every candidate (FP64: 32 x 32 and 64 x 32 tiles; split:
+/* Autotune the schedule of `mode`: every candidate (FP64: warp tiles of 8 and 16 rows; split:
  * stacking on and off) runs on these operands (c_dev is overwritten), timed with CUDA events
  * on `stream`, and the fastest is kept. The choice is cached per device and block-structure
  * signature for the life of the process; a plan with the same signature takes it without

@@ -300,21 +300,11 @@ __global__ void __launch_bounds__(256) k_pack_a(const double* __restrict__ scr, 
   }
 }
 
-// Element (r, c) of a B operand block: the block itself (k x n row-major), or for a complex
-// block (k x n complex, interleaved) its real 2k x 2n form of 2 x 2 blocks [[Re, Im], [-Im, Re]].
-template <bool CPLX>
-__device__ __forceinline__ double b_elem(const double* __restrict__ blk, int64_t r, int c, int cols) {
-  if constexpr (!CPLX) return __ldg(blk + r * cols + c);
-  const double v = __ldg(blk + (r >> 1) * cols + (c & ~1) + ((r ^ c) & 1));
-  return ((r & 1) && !(c & 1)) ? -v : v;
-}
-
 // Column scales and slices of B (k x n row-major), one CTA per (operand block, 32-column
 // tile). Phase 1: thread (row group g, column c) folds rows g, g + 8, ... of its column (a
 // warp reads 32 consecutive columns of one row); the 8 partial maxima per column meet in
 // shared memory. Phase 2: one thread per 16-byte chunk (8 consecutive k of one column) of
 // every 64-wide k tile writes the chunk of every slice plane.
-template <bool CPLX>
 __global__ void __launch_bounds__(256) k_pack_b_cols(const double* __restrict__ scr, const double* __restrict__ src,
                                                      const SplitOperand* __restrict__ ops,
                                                      const int2* __restrict__ col_tiles, int ntiles,
@@ -334,12 +324,7 @@ __global__ void __launch_bounds__(256) k_pack_b_cols(const double* __restrict__ 
       for (int r = g; r < o.rows; r += 32) {
         double v[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if constexpr (CPLX)
-            v[u] = r + 8 * u < o.rows ? b_elem<true>(blk, r + 8 * u, c0 + lane, o.cols) : 0.0;
-          else
-            v[u] = r + 8 * u < o.rows ? __ldg(col + (int64_t)(r + 8 * u) * o.cols) : 0.0;
-        }
+        for (int u = 0; u < 4; ++u) v[u] = r + 8 * u < o.rows ? __ldg(col + (int64_t)(r + 8 * u) * o.cols) : 0.0;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const uint32_t h = (uint32_t)__double2hiint(v[u]) & 0x7FFFFFFFu;
@@ -377,18 +362,107 @@ __global__ void __launch_bounds__(256) k_pack_b_cols(const double* __restrict__ 
       uint32_t sg[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        double x = 0.0;
-        if (k0 + j < o.rows) {
-          if constexpr (CPLX) x = b_elem<true>(blk, k0 + j, c0 + cc, o.cols);
-          else x = col[(k0 + j) * o.cols];
-        }
-        y[j] = digits_of(x, e, sg[j]);
+        y[j] = digits_of(k0 + j < o.rows ? col[(k0 + j) * o.cols] : 0.0, e, sg[j]);
       }
       // tile layout [ks][slice][n_core][k_core][8 columns x 16 B]: the slices of a 16-wide k
       // step form one 192-row K-major operand (slice q = rows 32 (q-1) .. 32 q - 1)
       const int64_t tile = (int64_t)tt.y * o.ktiles + kt;
       store_planes(y, sg, pack + o.pack_off + tile * (int64_t)(kS * kBTile) + (int64_t)ks * (kS * 1024) + n_core * 256 +
                               k_core * 128 + n8 * 16, 1024);
+    }
+    __syncthreads();   // smx / se are rewritten by the next column tile
+  }
+}
+
+// The slice planes of two columns of a complex block's real form, four rows of it (8 real k):
+// y[2 r] and y[2 r + 1] hold the digits of Re and Im of row r; the first column is (Re, -Im, ..),
+// the second, 16 bytes on, (Im, Re, ..).
+template <int P>
+__device__ __forceinline__ void store_plane_cplx(const uint64_t* y, const uint32_t* s0, const uint32_t* s1, uint8_t* dst) {
+  uint32_t f[8], v[4], w[4];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) f[j] = __float_as_uint(digit_value<P>(y[j]));
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    v[r] = __byte_perm(f[2 * r], f[2 * r + 1], 0x7632) ^ s0[r];
+    w[r] = __byte_perm(f[2 * r + 1], f[2 * r], 0x7632) ^ s1[r];
+  }
+  *reinterpret_cast<uint4*>(dst + P * 1024) = make_uint4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<uint4*>(dst + P * 1024 + 16) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// The same for a complex B block (k x n complex, interleaved) as its real 2k x 2n form of 2 x 2
+// blocks [[Re, Im], [-Im, Re]]: an element's two columns have the same scale and the same digits
+// up to sign, so each element is read once per phase (16 bytes) and sliced once. A thread takes 4
+// rows of one complex column. Hubbard, D = 3000: 23.5 -> 16.9
+// us against reading and slicing every element of the real form for itself.
+__global__ void __launch_bounds__(256) k_pack_b_cplx(const double* __restrict__ scr, const double* __restrict__ src,
+                                                     const SplitOperand* __restrict__ ops,
+                                                     const int2* __restrict__ col_tiles, int ntiles,
+                                                     int32_t* __restrict__ exps, uint8_t* __restrict__ pack) {
+  constexpr int kC = kTN / 2;   // complex columns of a tile
+  __shared__ uint32_t smx[16][kC], snz[16][kC];
+  __shared__ int se[kC];
+  const int c = threadIdx.x & (kC - 1), g = threadIdx.x / kC;
+  for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
+    const int2 tt = col_tiles[ti];
+    const SplitOperand o = ops[tt.x];
+    const int rows = o.rows >> 1, stride = o.cols >> 1;   // complex rows and columns
+    const int nc = min(kC, stride - tt.y * kC);
+    const double2* col = reinterpret_cast<const double2*>(operand_block(scr, src, o.src_off)) + tt.y * kC + c;
+    uint32_t mx = 0, nz = 0;   // largest high word of |Re| and |Im|, any nonzero bit
+    if (c < nc) {
+      for (int r = g; r < rows; r += 64) {
+        double2 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = r + 16 * u < rows ? __ldg(col + (int64_t)(r + 16 * u) * stride) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t a = (uint32_t)__double2hiint(v[u].x) & 0x7FFFFFFFu, b = (uint32_t)__double2hiint(v[u].y) & 0x7FFFFFFFu;
+          mx = max(mx, max(a, b));
+          nz |= a | b | (uint32_t)__double2loint(v[u].x) | (uint32_t)__double2loint(v[u].y);
+        }
+      }
+    }
+    smx[g][c] = mx;
+    snz[g][c] = nz;
+    __syncthreads();
+    if (threadIdx.x < kC) {
+      uint32_t m = 0, z = 0;
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        m = max(m, smx[q][c]);
+        z |= snz[q][c];
+      }
+      const int f = z ? max(1, (int)(m >> 20)) : 0;
+      se[c] = exp_of_field(f);
+      if (c < nc) exps[o.exp_off + tt.y * kTN + 2 * c] = exps[o.exp_off + tt.y * kTN + 2 * c + 1] = f;
+    }
+    __syncthreads();
+    const int e = se[c];
+    uint8_t* tile = pack + o.pack_off + (int64_t)tt.y * o.ktiles * (kS * kBTile) + (c >> 2) * 256 + (c & 3) * 32;
+    // items: (8 real k) x (complex column), 16 columns side by side
+    for (int r0 = 4 * g; r0 < rows; r0 += 64) {
+      if (c >= nc) break;       // padding: the buffer was zeroed once
+      uint64_t y[8];
+      uint32_t s0[4], s1[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const double2 x = r0 + r < rows ? col[(int64_t)(r0 + r) * stride] : make_double2(0.0, 0.0);
+        uint32_t a, b;
+        y[2 * r] = digits_of(x.x, e, a);
+        y[2 * r + 1] = digits_of(x.y, e, b);
+        s0[r] = a | ((b ^ 0x8000u) << 16);
+        s1[r] = b | (a << 16);
+      }
+      const int k8 = r0 >> 2;   // 16-byte chunk along k: two to a 16-wide step
+      uint8_t* dst = tile + (int64_t)(k8 >> 1) * (kS * 1024) + (k8 & 1) * 128;
+      store_plane_cplx<0>(y, s0, s1, dst);
+      store_plane_cplx<1>(y, s0, s1, dst);
+      store_plane_cplx<2>(y, s0, s1, dst);
+      store_plane_cplx<3>(y, s0, s1, dst);
+      store_plane_cplx<4>(y, s0, s1, dst);
+      store_plane_cplx<5>(y, s0, s1, dst);
     }
     __syncthreads();   // smx / se are rewritten by the next column tile
   }
@@ -1282,13 +1356,13 @@ void SplitPlan::build(const CtrctPlan& p, cudaStream_t s) {
     }
     QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pack_a, 256, 0));
     // four waves: CTAs of one wave finish up to a quarter apart (their ranges differ in locality).
-    // k_pack_a: see there; k_pack_b_cols, complex Hubbard: 27 -> 23.5 us
+    // k_pack_a: see there; B, complex Hubbard: 27 -> 23.5 us
     pack_a_grid = (int)std::max<int64_t>(1, std::min<int64_t>((n_a_pchunks + 255) / 256,
                                                               (int64_t)std::max(1, per_sm) * p.ctx->num_sms * 4));
     if (p.a.dtype == QLTG_C128)
-      QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pack_b_cols<true>, 256, 0));
+      QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pack_b_cplx, 256, 0));
     else
-      QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pack_b_cols<false>, 256, 0));
+      QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pack_b_cols, 256, 0));
     pack_b_grid = std::max(1, std::min((int)b_col_tiles.size(), std::max(1, per_sm) * p.ctx->num_sms * 4));
   }
   d_a_ops = upload(a_ops, s);
@@ -1353,11 +1427,11 @@ void pack_split_operand(SplitPlan& sp, bool side_a, const void* scratch, const v
     }
     const int nt = (int)sp.b_col_tiles.size();
     if (sp.b_ops[0].cplx)
-      k_pack_b_cols<true><<<sp.pack_b_grid, 256, 0, s>>>(X, Xs, sp.d_b_ops.as<SplitOperand>(),
+      k_pack_b_cplx<<<sp.pack_b_grid, 256, 0, s>>>(X, Xs, sp.d_b_ops.as<SplitOperand>(),
                                                          sp.d_b_col_tiles.as<int2>(), nt, sp.b_exps.as<int32_t>(),
                                                          sp.b_packed.as<uint8_t>());
     else
-      k_pack_b_cols<false><<<sp.pack_b_grid, 256, 0, s>>>(X, Xs, sp.d_b_ops.as<SplitOperand>(),
+      k_pack_b_cols<<<sp.pack_b_grid, 256, 0, s>>>(X, Xs, sp.d_b_ops.as<SplitOperand>(),
                                                           sp.d_b_col_tiles.as<int2>(), nt, sp.b_exps.as<int32_t>(),
                                                           sp.b_packed.as<uint8_t>());
   }

@@ -57,3 +57,29 @@ def test_digits(gpu, m, k, n, kind):
     bound = ((4.6 * k + 6 * -(-k // 160)) * 2.0**-47 * np.abs(A).max(1)[:, None] * np.abs(B).max(0)
              + -(-k // 1920) * 2.0**-52 * np.abs(exact))
     assert np.all(np.abs(C - exact) <= bound), float((np.abs(C - exact) / bound).max())
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 1, 9), (33, 3, 15), (130, 9, 16), (7, 63, 17), (40, 64, 33), (5, 66, 48), (129, 81, 10)])
+def test_digits_complex(gpu, m, k, n):
+    """Complex operands (B sliced as its real 2k x 2n form): column remainders of the 16-column
+    tiles, row remainders of the 4-row pieces. Integers, and halves of them on one side in every
+    third row, so rows and columns have different scales: the results are exact."""
+    rng = np.random.default_rng(m + 10 * k + n)
+
+    def ints(*shape):
+        x = rng.integers(-90, 91, shape) + 1j * rng.integers(-90, 91, shape)
+        x[::3] *= 0.5
+        return x
+
+    A, B = ints(m, k), ints(k, n)
+    B[:, n // 2] = 0
+    B[:, n - 1] = B[:, n - 1].real
+    leg = lambda d, direction: Leg(direction, np.asarray([[0]]), np.asarray([d]))
+    inner = leg(k, OUT)
+    one = np.asarray([[0, 0]])
+    a = BSTensor([leg(m, IN), inner], one, np.complex128, A.ravel())
+    b = BSTensor([inner.inverse(), leg(n, OUT)], one, np.complex128, B.ravel())
+    plan = ContractionPlan(a, b, [[1], [0]])
+    c = plan.execute(DTensor.from_host(a), DTensor.from_host(b), mode="split")
+    plan.device_status()
+    assert np.array_equal(c.to_host().to_dense(), A @ B)

@@ -42,33 +42,64 @@ struct LincombArgs {
   T coef[kLincombMax + 1];
 };
 
-__device__ __forceinline__ double lc_mul(double a, double x) { return a * x; }
+__device__ __forceinline__ double lc_mul(double a, double x) { return __dmul_rn(a, x); }
 __device__ __forceinline__ double2 lc_mul(double2 a, double2 x) {
   return make_double2(fma(a.x, x.x, -a.y * x.y), fma(a.x, x.y, a.y * x.x));
 }
-__device__ __forceinline__ double lc_add(double a, double b) { return a + b; }
-__device__ __forceinline__ double2 lc_add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double lc_zero(double) { return 0.0; }
-__device__ __forceinline__ double2 lc_zero(double2) { return make_double2(0.0, 0.0); }
+// v + (a x), rounded twice as the reference's scaled copies and additions are
+__device__ __forceinline__ double lc_add(double v, double ax) { return __dadd_rn(v, ax); }
+__device__ __forceinline__ double2 lc_add(double2 v, double2 ax) { return make_double2(__dadd_rn(v.x, ax.x), __dadd_rn(v.y, ax.y)); }
 
 // `out` may be one of the source buffers (in-place LinearCombine / AddScaledAssign: the same
 // layout, so each element is read and written by one thread at the same position); it is
 // therefore not declared __restrict__.
+// A thread takes up to four elements side by side (as many as its warp has, by branches: an FP64
+// instruction costs a warp the same, 68 - 80 cycles, with every lane off): the lists are read once
+// for them and their loads are in flight together. A product and a sum per contribution: 8 vectors
+// cost the FP64 pipe 24 us per 744k elements, their bytes 8 us. Where a plan has fewer items than the
+// GPU holds CTAs, four CTAs share one (shift 2). 8 vectors
+// of 70k / 744k / 2.0M elements: 59 / 64 / 71 -> 13 / 35 / 67 us.
+template <typename T, int U>
+__device__ __forceinline__ void lc_elements(const LincombItem& w, const LincombSrc* __restrict__ srcs,
+                                            const LincombArgs<T>& args, int e0, T* out) {
+  T v[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) v[u] = T{};
+  for (int c = w.c0; c < w.c1; ++c) {
+    const LincombSrc s = srcs[c];
+    const T a = args.coef[s.t];
+    const T* x = args.src[s.t] + s.off;
+    T y[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) y[u] = e0 + 256 * u < w.n ? x[e0 + 256 * u] : T{};
+    if (c == w.c0) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = lc_mul(a, y[u]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = lc_add(v[u], lc_mul(a, y[u]));
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (e0 + 256 * u < w.n) out[w.out_off + e0 + 256 * u] = v[u];
+}
+
 template <typename T>
-__global__ void __launch_bounds__(256) k_lincomb(const LincombItem* __restrict__ items, int nitems,
+__global__ void __launch_bounds__(256) k_lincomb(const LincombItem* __restrict__ items, int nitems, int shift,
                                                  const LincombSrc* __restrict__ srcs,
                                                  const __grid_constant__ LincombArgs<T> args,
                                                  T* out) {
-  for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-    const LincombItem w = items[it];
-    for (int e = threadIdx.x; e < w.n; e += blockDim.x) {
-      T v = lc_zero(T());
-      for (int c = w.c0; c < w.c1; ++c) {
-        const LincombSrc s = srcs[c];
-        const T x = lc_mul(args.coef[s.t], args.src[s.t][s.off + e]);
-        v = c == w.c0 ? x : lc_add(v, x);
-      }
-      out[w.out_off + e] = v;
+  const int part = kLincombChunk >> shift;
+  for (int it = blockIdx.x; it < nitems << shift; it += gridDim.x) {
+    const LincombItem w = items[it >> shift];
+    const int b0 = (it & ((1 << shift) - 1)) * part;
+    for (int b = b0; b < min(w.n, b0 + part); b += 1024) {
+      const int e0 = b + threadIdx.x, left = w.n - (e0 & ~31);   // of the warp's first element on
+      if (left > 768) lc_elements<T, 4>(w, srcs, args, e0, out);
+      else if (left > 512) lc_elements<T, 3>(w, srcs, args, e0, out);
+      else if (left > 256) lc_elements<T, 2>(w, srcs, args, e0, out);
+      else if (left > 0) lc_elements<T, 1>(w, srcs, args, e0, out);
     }
   }
 }
@@ -223,7 +254,9 @@ int qltg_lincomb_exec(qltg_lincomb_plan* plan, const void* const* tens_dev, cons
                "result expanded to new blocks cannot be written in place");
     const int ni = (int)plan->items.size();
     if (!ni) return;
-    const int grid = std::min(ni, std::max(1, plan->ctx->num_sms) * 8);
+    const int wave = std::max(1, plan->ctx->num_sms) * 8;
+    const int shift = ni < wave ? 2 : 0;
+    const int grid = std::min(ni << shift, 4 * wave);   // not one wave: equal shares leave a ragged end
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (plan->out.dtype == QLTG_C128) {
       LincombArgs<double2> a{};
@@ -233,7 +266,7 @@ int qltg_lincomb_exec(qltg_lincomb_plan* plan, const void* const* tens_dev, cons
       }
       a.src[kLincombMax] = static_cast<const double2*>(res_dev);
       a.coef[kLincombMax] = make_double2(plan->coefs[2 * n], plan->coefs[2 * n + 1]);
-      k_lincomb<double2><<<grid, 256, 0, s>>>(plan->d_items.as<LincombItem>(), ni, plan->d_srcs.as<LincombSrc>(), a,
+      k_lincomb<double2><<<grid, 256, 0, s>>>(plan->d_items.as<LincombItem>(), ni, shift, plan->d_srcs.as<LincombSrc>(), a,
                                               static_cast<double2*>(out_dev));
     } else {
       LincombArgs<double> a{};
@@ -243,7 +276,7 @@ int qltg_lincomb_exec(qltg_lincomb_plan* plan, const void* const* tens_dev, cons
       }
       a.src[kLincombMax] = static_cast<const double*>(res_dev);
       a.coef[kLincombMax] = plan->coefs[2 * n];
-      k_lincomb<double><<<grid, 256, 0, s>>>(plan->d_items.as<LincombItem>(), ni, plan->d_srcs.as<LincombSrc>(), a,
+      k_lincomb<double><<<grid, 256, 0, s>>>(plan->d_items.as<LincombItem>(), ni, shift, plan->d_srcs.as<LincombSrc>(), a,
                                              static_cast<double*>(out_dev));
     }
     QLTG_CUDA(cudaGetLastError());

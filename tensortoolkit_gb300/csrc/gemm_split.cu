@@ -393,9 +393,11 @@ __device__ __forceinline__ void store_plane_cplx(const uint64_t* y, const uint32
 
 // The same for a complex B block (k x n complex, interleaved) as its real 2k x 2n form of 2 x 2
 // blocks [[Re, Im], [-Im, Re]]: an element's two columns have the same scale and the same digits
-// up to sign, so each element is read once per phase (16 bytes) and sliced once. A thread takes 4
-// rows of one complex column. Hubbard, D = 3000: 23.5 -> 16.9
-// us against reading and slicing every element of the real form for itself.
+// up to sign, so each element is read once per phase and sliced once: 16 bytes at a time where the
+// operand lies on 16 bytes (WIDE), else its two parts (a caller's buffer may be any range of real
+// values). A thread takes 4 rows of one complex column. Hubbard, D = 3000: 23.5 -> 16.9 us against
+// reading and slicing every element of the real form for itself.
+template <bool WIDE>
 __global__ void __launch_bounds__(256) k_pack_b_cplx(const double* __restrict__ scr, const double* __restrict__ src,
                                                      const SplitOperand* __restrict__ ops,
                                                      const int2* __restrict__ col_tiles, int ntiles,
@@ -407,15 +409,20 @@ __global__ void __launch_bounds__(256) k_pack_b_cplx(const double* __restrict__ 
   for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
     const int2 tt = col_tiles[ti];
     const SplitOperand o = ops[tt.x];
-    const int rows = o.rows >> 1, stride = o.cols >> 1;   // complex rows and columns
-    const int nc = min(kC, stride - tt.y * kC);
-    const double2* col = reinterpret_cast<const double2*>(operand_block(scr, src, o.src_off)) + tt.y * kC + c;
+    const int rows = o.rows >> 1;   // complex rows
+    const int nc = min(kC, (o.cols >> 1) - tt.y * kC);
+    const double* col = operand_block(scr, src, o.src_off) + 2 * (tt.y * kC + c);
+    auto element = [&](int r) -> double2 {
+      const double* x = col + (int64_t)r * o.cols;
+      if constexpr (WIDE) return __ldg(reinterpret_cast<const double2*>(x));
+      else return make_double2(__ldg(x), __ldg(x + 1));
+    };
     uint32_t mx = 0, nz = 0;   // largest high word of |Re| and |Im|, any nonzero bit
     if (c < nc) {
       for (int r = g; r < rows; r += 64) {
         double2 v[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = r + 16 * u < rows ? __ldg(col + (int64_t)(r + 16 * u) * stride) : make_double2(0.0, 0.0);
+        for (int u = 0; u < 4; ++u) v[u] = r + 16 * u < rows ? element(r + 16 * u) : make_double2(0.0, 0.0);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const uint32_t a = (uint32_t)__double2hiint(v[u].x) & 0x7FFFFFFFu, b = (uint32_t)__double2hiint(v[u].y) & 0x7FFFFFFFu;
@@ -448,7 +455,7 @@ __global__ void __launch_bounds__(256) k_pack_b_cplx(const double* __restrict__ 
       uint32_t s0[4], s1[4];
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        const double2 x = r0 + r < rows ? col[(int64_t)(r0 + r) * stride] : make_double2(0.0, 0.0);
+        const double2 x = r0 + r < rows ? element(r0 + r) : make_double2(0.0, 0.0);
         uint32_t a, b;
         y[2 * r] = digits_of(x.x, e, a);
         y[2 * r + 1] = digits_of(x.y, e, b);
@@ -1360,7 +1367,7 @@ void SplitPlan::build(const CtrctPlan& p, cudaStream_t s) {
     pack_a_grid = (int)std::max<int64_t>(1, std::min<int64_t>((n_a_pchunks + 255) / 256,
                                                               (int64_t)std::max(1, per_sm) * p.ctx->num_sms * 4));
     if (p.a.dtype == QLTG_C128)
-      QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pack_b_cplx, 256, 0));
+      QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pack_b_cplx<true>, 256, 0));
     else
       QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pack_b_cols, 256, 0));
     pack_b_grid = std::max(1, std::min((int)b_col_tiles.size(), std::max(1, per_sm) * p.ctx->num_sms * 4));
@@ -1426,14 +1433,17 @@ void pack_split_operand(SplitPlan& sp, bool side_a, const void* scratch, const v
       return;
     }
     const int nt = (int)sp.b_col_tiles.size();
-    if (sp.b_ops[0].cplx)
-      k_pack_b_cplx<<<sp.pack_b_grid, 256, 0, s>>>(X, Xs, sp.d_b_ops.as<SplitOperand>(),
-                                                         sp.d_b_col_tiles.as<int2>(), nt, sp.b_exps.as<int32_t>(),
-                                                         sp.b_packed.as<uint8_t>());
-    else
+    if (sp.b_ops[0].cplx) {
+      // (blocks lie whole elements apart)
+      const bool wide = ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Xs)) & 15) == 0;
+      auto* kernel = wide ? k_pack_b_cplx<true> : k_pack_b_cplx<false>;
+      kernel<<<sp.pack_b_grid, 256, 0, s>>>(X, Xs, sp.d_b_ops.as<SplitOperand>(), sp.d_b_col_tiles.as<int2>(), nt,
+                                            sp.b_exps.as<int32_t>(), sp.b_packed.as<uint8_t>());
+    } else {
       k_pack_b_cols<<<sp.pack_b_grid, 256, 0, s>>>(X, Xs, sp.d_b_ops.as<SplitOperand>(),
                                                           sp.d_b_col_tiles.as<int2>(), nt, sp.b_exps.as<int32_t>(),
                                                           sp.b_packed.as<uint8_t>());
+    }
   }
   QLTG_CUDA(cudaGetLastError());
   (side_a ? sp.a_ready : sp.b_ready) = true;

@@ -7,8 +7,10 @@
  * blocks in ascending block index, each block row-major over its degeneracy dims, at
  * cumulative offsets (reference qltensor/blk_spar_data_ten/blk_spar_data_ten.h:53-572,
  * data_blk_operations.h:137-145). Complex data is interleaved (re, im) doubles, i.e.
- * std::complex<double>. Streams are passed as `void*` (a cudaStream_t, NULL = legacy
- * default stream).
+ * std::complex<double>. Complex buffers lie on 16 bytes: a call whose kernels would read or
+ * write whole elements of one that does not returns QLTG_ERR_INVALID (split precision works on
+ * real values, and takes one where nothing is transposed and no output block is skinny).
+ * Streams are passed as `void*` (a cudaStream_t, NULL = legacy default stream).
  *
  * Ownership: callers own every tensor buffer they pass in. The library owns plans,
  * workspaces, CUDA graphs and the outputs of decompositions (freed with the matching

@@ -229,6 +229,7 @@ int qltg_accum_exec(qltg_accum_plan* plan, const void* a_dev, const void* b_dev,
     QLTG_CHECK(c_out_dev != a_dev && c_out_dev != b_dev, QLTG_ERR_INVALID, "output aliases an input");
     QLTG_CHECK(!(plan->expanded && c_in_dev && c_out_dev == c_in_dev), QLTG_ERR_INVALID,
                "an expanded output cannot be written over the input output");
+    if (!plan->items.empty()) check_aligned(plan->out.elem_bytes(), {beta_zero ? nullptr : c_in_dev, c_out_dev});
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (plan->ctr.c.size > 0) exec_contraction(plan->ctr, a_dev, b_dev, plan->t_buf.get(), mode, s);
     const int ni = (int)plan->items.size();

@@ -122,6 +122,7 @@ void axis_scale(qltg_ctx* ctx, const Meta& m, int axis, const std::vector<double
                 const double* alpha, const double* beta, cudaStream_t s) {
   if (m.nblk == 0) return;
   QLTG_CHECK(in && out, QLTG_ERR_INVALID, "null buffer");
+  check_aligned(m.elem_bytes(), {in, out});
   const bool cplx = m.dtype == QLTG_C128;
   QLTG_CHECK(cplx || (alpha[1] == 0.0 && beta[1] == 0.0), QLTG_ERR_INVALID, "complex alpha or beta for a real tensor");
   const auto items = axis_items(m, axis);
@@ -456,6 +457,7 @@ int qltg_axis_monomial_exec(qltg_axis_plan* plan, const void* in_dev, void* out_
     QLTG_CHECK(in_dev != out_dev, QLTG_ERR_INVALID, "output aliases the input");
     QLTG_CUDA(cudaSetDevice(plan->ctx->device));
     if (!plan->mono_items) return;
+    check_aligned(plan->mono_out.elem_bytes(), {in_dev, out_dev});
     const bool cplx = plan->mono_out.dtype == QLTG_C128;
     QLTG_CHECK(cplx || (alpha[1] == 0.0 && beta[1] == 0.0), QLTG_ERR_INVALID, "complex alpha or beta for a real tensor");
     cudaStream_t s = static_cast<cudaStream_t>(stream);

@@ -235,6 +235,8 @@ void exec_contraction(CtrctPlan& p, const void* a, const void* b, void* c, int m
     op.b = p.b_t.get();
   }
   if (stage == 1) return;
+  // the FP64 kernels work on whole elements; the slices of split precision are made from FP64 values
+  check_aligned(mode == QLTG_MODE_FP64 || !p.sched.skinny.empty() ? eb : sizeof(double), {a, b, c});
   if (mode == QLTG_MODE_FP64)
     launch_gemm_f64(p.sched, op, c, p.a.dtype == QLTG_C128, p.ctx->num_sms, s);
   else

@@ -254,6 +254,8 @@ int qltg_lincomb_exec(qltg_lincomb_plan* plan, const void* const* tens_dev, cons
                "result expanded to new blocks cannot be written in place");
     const int ni = (int)plan->items.size();
     if (!ni) return;
+    check_aligned(plan->out.elem_bytes(), {plan->used[n] ? res_dev : nullptr, out_dev});
+    for (int i = 0; i < n; ++i) check_aligned(plan->out.elem_bytes(), {plan->used[i] ? tens_dev[i] : nullptr});
     const int wave = std::max(1, plan->ctx->num_sms) * 8;
     const int shift = ni < wave ? 2 : 0;
     const int grid = std::min(ni << shift, 4 * wave);   // not one wave: equal shares leave a ragged end

@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <cstring>
+#include <initializer_list>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -101,6 +102,14 @@ class DevBuf {
   size_t n_ = 0;
   bool own_ = true;
 };
+
+// A buffer that kernels read or write in whole elements lies on a multiple of their size (16 bytes
+// for complex128): anything else would be a misaligned access on the GPU. Null is left alone.
+inline void check_aligned(size_t elem_bytes, std::initializer_list<const void*> bufs) {
+  for (const void* p : bufs)
+    QLTG_CHECK(reinterpret_cast<uintptr_t>(p) % elem_bytes == 0, QLTG_ERR_INVALID,
+               "buffer is not aligned to its " + std::to_string(elem_bytes) + "-byte elements");
+}
 
 // Streaming multiprocessors of the current device (grid sizing for kernels launched without
 // a context at hand).

@@ -338,6 +338,7 @@ int64_t plan_block(PermDesc& d, int m, const int64_t* dd, const int64_t* ds, int
 template <typename T>
 void launch_permute(const PermDesc* descs, int64_t nblocks, const int32_t* item_block, int64_t nitems, const void* src,
                     void* dst, cudaStream_t s) {
+  check_aligned(sizeof(T), {src, dst});
   const unsigned grid = (unsigned)std::min<int64_t>((nitems + kPermWarps - 1) / kPermWarps,
                                                     (int64_t)current_sm_count() * kPermCtasPerSm);
   k_permute<T><<<grid, kPermThreads, 0, s>>>(descs, (int)nblocks, item_block, nitems, static_cast<const T*>(src),

@@ -1,11 +1,13 @@
 """Complex tensors whose buffer starts at 8 modulo 16 bytes (any range of a float64 tensor): split
-precision reads real values where nothing has to be transposed and no output block is skinny. Small
-integers, so the result must equal numpy's bit for bit."""
+precision reads real values where nothing has to be transposed and no output block is skinny (small
+integers, so the result must equal numpy's bit for bit); what works on whole elements refuses them."""
 import numpy as np
 import pytest
 import torch
 
+from tensortoolkit_gb300 import api
 from tensortoolkit_gb300.api import ContractionPlan, DTensor
+from tensortoolkit_gb300.capi import QltgError
 from tensortoolkit_gb300.tensor import IN, OUT, BSTensor, Leg
 
 pytestmark = pytest.mark.gpu
@@ -44,3 +46,30 @@ def test_split_reads_real_values(gpu, m, k, n):
         c = plan.execute(x, y, out, mode="split")
         plan.device_status()
         assert np.array_equal(c.to_host().to_dense(), a.to_dense() @ b.to_dense())
+
+
+def test_whole_elements_refuse(gpu):
+    a, b = _matrices(40, 24, 33)
+    x, y = _at_8(a), _at_8(b)
+    good_a, good_b = DTensor.from_host(a), DTensor.from_host(b)
+    sa, sb = _matrices(24, 5, 6)   # k = 5, n = 6: a skinny block
+    plan = ContractionPlan(a, b, [[1], [0]])
+    out = plan.execute(good_a, good_b)
+    skinny = ContractionPlan(sa, sb, [[1], [0]])
+    swapped = api.TransposePlan(b, [1, 0])
+    b_t = swapped.execute(good_b).to_host()
+    transposing = ContractionPlan(a, b_t, [[1], [1]])
+    refused = [lambda: plan.execute(x, good_b), lambda: plan.execute(good_a, y),
+               lambda: plan.execute(good_a, good_b, _at_8(out.to_host())),
+               lambda: skinny.execute(_at_8(sa), DTensor.from_host(sb), mode="split"),
+               lambda: transposing.execute(good_a, _at_8(b_t), mode="split"),
+               lambda: swapped.execute(y), lambda: api.Transpose(y, [1, 0]),
+               lambda: api.LinearCombine([1.0, 2.0], [good_a, x]), lambda: api.AddScaledAssign(x, 2.0, good_a),
+               lambda: api.ApplyAxisDiagonal(x, 0, np.ones(40)),
+               lambda: api.ContractTailHeadContiguousAccumulate(good_a, good_b, 1, 0, 1, 1.0, 1.0, _at_8(out.to_host())),
+               lambda: api.SVD(x, 1, [0], 0.0, 1, 40), lambda: api.QR(x, 1, [0])]
+    for call in refused:
+        with pytest.raises(QltgError, match="16-byte elements"):
+            call()
+    # nothing ran, the context is as it was
+    assert np.array_equal(plan.execute(good_a, good_b).to_host().data, out.to_host().data)

@@ -78,10 +78,10 @@ struct GemmTileRun {
   int32_t tm0, tn0, tn_count;
 };
 // Skinny output blocks (n, k <= 8): a piece of a block's m x n outputs (skinny_outputs of them from
-// o0) and the block's entries [e0, e1), its tasks' k values laid end to end: the A column (element
+// pass p0 of 128 outputs on) and the block's entries [e0, e1), its tasks' k values laid end to end: the A column (element
 // (row) at a_off + row a_rs) and the B row (n values at b_off) that each multiplies.
 struct SkinnyItem {
-  int32_t cblk, o0, e0, e1;
+  int32_t cblk, p0, e0, e1;
 };
 struct SkinnyEntry {
   int64_t a_off, b_off;        // | kFromSrc
@@ -108,6 +108,7 @@ struct GemmSchedule {
   std::vector<SkinnyItem> skinny;       // pieces of skinny blocks (n, k <= 8)
   std::vector<SkinnyEntry> skinny_entry;
   int skinny_outputs = 128;             // outputs of an item (the last of a block may have fewer)
+  bool skinny_long = false;             // some block's outputs need 64-bit positions
   DevBuf lists;                          // holds the device copies below (parts of it)
   DevBuf d_cblk, d_task, d_run, d_skinny, d_entry, d_counter;
   int bm = 32;                          // rows of the FP64 tiles of a CTA's four warps

@@ -69,10 +69,11 @@ void set_f64_tile(CtrctPlan& p, int bm, cudaStream_t s) {
 // to add under a quarter of empty ones, an item stands for four passes, to keep the list short.
 static void skinny_list(GemmSchedule& g, int num_sms) {
   int64_t passes = 0, items = 0;
+  g.skinny_long = false;
   for (int32_t q = 0; q < (int32_t)g.cblk.size(); ++q) {
     if (!skinny_cblk(g, q)) continue;
     const int64_t outputs = (int64_t)g.cblk[q].m * g.cblk[q].n;
-    QLTG_CHECK(outputs < ((int64_t)1 << 31) - 512, QLTG_ERR_UNSUPPORTED, "output block too large");
+    g.skinny_long |= outputs >= ((int64_t)1 << 31) - 512;   // (a pass counts on past the block's end)
     passes += (outputs + 127) / 128;
     items += (outputs + 511) / 512;
   }
@@ -89,7 +90,7 @@ static void skinny_list(GemmSchedule& g, int num_sms) {
     }
     QLTG_CHECK(g.skinny_entry.size() < ((size_t)1 << 31), QLTG_ERR_UNSUPPORTED, "too many small tasks");
     for (int64_t o = 0; o < (int64_t)cb.m * cb.n; o += g.skinny_outputs)
-      g.skinny.push_back(SkinnyItem{q, (int32_t)o, (int32_t)e0, (int32_t)g.skinny_entry.size()});
+      g.skinny.push_back(SkinnyItem{q, (int32_t)(o / 128), (int32_t)e0, (int32_t)g.skinny_entry.size()});
   }
 }
 

@@ -225,20 +225,21 @@ __device__ __forceinline__ void fold_field(unsigned mask, int key, int v, int32_
   if (key >= 0 && x > 0 && (int)(threadIdx.x & 31) == __ffs(m) - 1) atomicMax(fields + key, x);
 }
 
-// Outputs o + lane + 32 u (u < U, clamped into the block) of one block, from all its entries.
-template <typename T, int U>
-__device__ __forceinline__ void skinny_pass(const GemmCBlk& cb, const SkinnyItem& item, int o, int lane,
+// Outputs o + lane + 32 u (u < U, clamped into the block) of one block, from all its entries. I: the
+// type of an output's position in its block.
+template <typename T, typename I, int U>
+__device__ __forceinline__ void skinny_pass(const GemmCBlk& cb, const SkinnyItem& item, I o, int lane,
                                             const SkinnyEntry* __restrict__ entry, const T* __restrict__ A,
                                             const T* __restrict__ As, const T* __restrict__ B, const T* __restrict__ Bs,
                                             T* __restrict__ C, const SkinnyFuse& fz, int32_t* __restrict__ fields) {
-  const int total = cb.m * cb.n;
+  const I total = (I)cb.m * cb.n;
   int row[U], col[U];
   T acc[U];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    const int x = min(o + 32 * u + lane, total - 1);
-    row[u] = x / cb.n;
-    col[u] = x - row[u] * cb.n;
+    const I x = min(o + 32 * u + lane, total - 1);
+    row[u] = (int)(x / cb.n);
+    col[u] = (int)(x - (I)row[u] * cb.n);
     acc[u] = zero_of(T());
   }
   int e = item.e0;
@@ -272,14 +273,16 @@ __device__ __forceinline__ void skinny_pass(const GemmCBlk& cb, const SkinnyItem
   }
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    const int x = o + 32 * u + lane;
+    const I x = o + 32 * u + lane;
     if (x < total) C[cb.c_off + x] = acc[u];
     // the outputs' order is that of the later operand's rows of k3 values
-    if (fz.exp_base >= 0) fold_field(0xffffffffu, x < total ? fz.exp_base + x / fz.k3 : -1, out_field(acc[u]), fields);
+    if (fz.exp_base >= 0) fold_field(0xffffffffu, x < total ? fz.exp_base + (int)(x / fz.k3) : -1, out_field(acc[u]), fields);
   }
 }
 
-template <typename T>
+// I = int64_t where a block has 2^31 outputs or more (17 GB of FP64 values); 64-bit divisions would
+// cost the others.
+template <typename T, typename I>
 __global__ void __launch_bounds__(kSkinnyThreads, sizeof(T) == 8 ? 7 : 5) k_gemm_skinny(
     const GemmCBlk* __restrict__ cblk, const SkinnyEntry* __restrict__ entry, const SkinnyItem* __restrict__ items,
     int npasses, int shift, const T* __restrict__ A, const T* __restrict__ As, const T* __restrict__ B,
@@ -290,16 +293,16 @@ __global__ void __launch_bounds__(kSkinnyThreads, sizeof(T) == 8 ? 7 : 5) k_gemm
   SkinnyItem next = items[it >> shift];
   for (; it < npasses; it += step) {
     const SkinnyItem item = next;
-    const int o = item.o0 + (it & ((1 << shift) - 1)) * kSkinnyPass;
+    const I o = (I)(item.p0 + (it & ((1 << shift) - 1))) * kSkinnyPass;
     if (it + step < npasses) next = items[(it + step) >> shift];
     const GemmCBlk cb = cblk[item.cblk];
-    const int left = cb.m * cb.n - o;
+    const I left = (I)cb.m * cb.n - o;
     if (left <= 0) continue;
     const SkinnyFuse fz = fuse ? fuse[item.cblk] : SkinnyFuse{-1, 1};
-    if (left > 96) skinny_pass<T, 4>(cb, item, o, lane, entry, A, As, B, Bs, C, fz, fields);
-    else if (left > 64) skinny_pass<T, 3>(cb, item, o, lane, entry, A, As, B, Bs, C, fz, fields);
-    else if (left > 32) skinny_pass<T, 2>(cb, item, o, lane, entry, A, As, B, Bs, C, fz, fields);
-    else skinny_pass<T, 1>(cb, item, o, lane, entry, A, As, B, Bs, C, fz, fields);
+    if (left > 96) skinny_pass<T, I, 4>(cb, item, o, lane, entry, A, As, B, Bs, C, fz, fields);
+    else if (left > 64) skinny_pass<T, I, 3>(cb, item, o, lane, entry, A, As, B, Bs, C, fz, fields);
+    else if (left > 32) skinny_pass<T, I, 2>(cb, item, o, lane, entry, A, As, B, Bs, C, fz, fields);
+    else skinny_pass<T, I, 1>(cb, item, o, lane, entry, A, As, B, Bs, C, fz, fields);
   }
 }
 
@@ -313,11 +316,11 @@ bool skinny_cblk(const GemmSchedule& g, int32_t q) {
   return true;
 }
 
-template <typename T>
+template <typename T, typename I>
 void launch_skinny(const GemmSchedule& g, const Operands& op, void* c, int grid, cudaStream_t s, const SkinnyFuse* fuse,
                    int32_t* fields) {
   const int shift = g.skinny_outputs == 4 * kSkinnyPass ? 2 : 0;
-  k_gemm_skinny<T><<<grid, kSkinnyThreads, 0, s>>>(
+  k_gemm_skinny<T, I><<<grid, kSkinnyThreads, 0, s>>>(
       g.d_cblk.as<GemmCBlk>(), g.d_entry.as<SkinnyEntry>(), g.d_skinny.as<SkinnyItem>(), (int)g.skinny.size() << shift,
       shift, static_cast<const T*>(op.a), static_cast<const T*>(op.a_src), static_cast<const T*>(op.b),
       static_cast<const T*>(op.b_src), static_cast<T*>(c), fuse, fields);
@@ -349,7 +352,7 @@ template <typename T>
 int skinny_wave(int num_sms) {
   static int per_sm = [] {
     int n = 0;
-    QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_gemm_skinny<T>, kSkinnyThreads, 0));
+    QLTG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_gemm_skinny<T, int32_t>, kSkinnyThreads, 0));
     return std::max(1, n);
   }();
   return std::max(1, num_sms) * per_sm;
@@ -370,8 +373,9 @@ void launch_gemm_f64_skinny(const GemmSchedule& g, const Operands& op, void* c, 
   const int ns = (int)g.skinny.size();
   if (!ns) return;
   const int grid = skinny_grid(ns, cplx, num_sms);
-  if (cplx) launch_skinny<double2>(g, op, c, grid, s, fuse, fields);
-  else launch_skinny<double>(g, op, c, grid, s, fuse, fields);
+  auto* launch = g.skinny_long ? (cplx ? launch_skinny<double2, int64_t> : launch_skinny<double, int64_t>)
+                               : (cplx ? launch_skinny<double2, int32_t> : launch_skinny<double, int32_t>);
+  launch(g, op, c, grid, s, fuse, fields);
   QLTG_CUDA(cudaGetLastError());
 }
 

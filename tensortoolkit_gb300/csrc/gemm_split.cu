@@ -718,9 +718,10 @@ __device__ __forceinline__ void drain_set(uint32_t lb, uint64_t (&z)[kDrainCols]
 // holds column c's eb.
 // Where no result can be subnormal or infinite (scales between 2^-450 and 2^450) and every |z| is
 // zero or has a bit in its high word, a product with 2^(lz - 1), which adds half an ulp at once,
-// puts the leading one at bit 62 (|z| < 2^62; a tie, which takes more than 53 bits, goes away from
-// zero): a third of the general form's instructions. Zeros are common: padding, and rows or
-// columns without data.
+// puts the leading one at bit 62 (|z| < 2^62); where that cleared the ten bits dropped it was a tie,
+// and the last bit kept goes, as in the general form (to even: an output must not depend on which
+// form its neighbours ask for). A third of the general form's instructions. Zeros are common:
+// padding, and rows or columns without data.
 __device__ __forceinline__ void fold_sums(const uint64_t (&z)[kDrainCols], int ea, int eb, bool neg, uint32_t tsum,
                                           bool add, double (&x)[kDrainCols]) {
   uint32_t low_only = 0;
@@ -744,8 +745,9 @@ __device__ __forceinline__ void fold_sums(const uint64_t (&z)[kDrainCols], int e
       const uint64_t lo = mad_wide((uint32_t)a[c], pow, 0x200u);
       const uint32_t mh = ah * pow + (uint32_t)(lo >> 32);
       const uint32_t hi = (mh >> 10) + __shfl_sync(0xffffffffu, kb, c) + (m * (1u << 20) + ka);
-      x[c] = __hiloint2double((int)((ah ? hi : 0u) | ((uint32_t)(z[c] >> 32) & 0x80000000u)),
-                              (int)__funnelshift_r((uint32_t)lo, mh, 10));
+      uint32_t w = __funnelshift_r((uint32_t)lo, mh, 10);
+      if (((uint32_t)lo & 0x3FFu) == 0) w &= ~1u;
+      x[c] = __hiloint2double((int)((ah ? hi : 0u) | ((uint32_t)(z[c] >> 32) & 0x80000000u)), (int)w);
     }
   } else {
 #pragma unroll

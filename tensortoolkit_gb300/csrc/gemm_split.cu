@@ -19,7 +19,8 @@
 //   has its own 128 x 32 FP32 accumulator in tensor memory (levels 2..7: 192 columns per set,
 //   two sets). Over 160 k the sums of levels 2..5 stay below 2^24 (level 5: 160 x 3 x 2^15) and
 //   are exact; level 6 may pass 2^24 by 1.1 and level 7 by 1.25 where every digit is at its
-//   limit, and then carry an FP32 rounding of one unit, 2^-48 or 2^-56. Every 160 k the drain
+//   limit and of one sign: the last 5 and 12 MMAs of the 160 k then round to multiples of two
+//   units (2^-48 and 2^-56; 8 units of 2^-48 in all measured there). Every 160 k the drain
 //   warps read the levels and fold them into one int64 per output (units 2^-50); at the end of
 //   a task C (+)= sign 2^(ea + eb - 50) z, rounded to FP64 with integer operations.
 // D = 4000 matvec against the seven-slice form: k_gemm_split 122 / 97 -> 98 / 90 us (steps 0 / 3),

@@ -55,11 +55,14 @@ enum { QLTG_IN = 0, QLTG_OUT = 1 };       /* TenIndexDirType */
  * QLTG_MODE_SPLIT: FP64 emulated with BF16 slices on the tcgen05 tensor cores: every row
  *                  of A / column of B is scaled by a power of two and rounded to six
  *                  balanced 8-bit digits, the 21 slice products of weight >= 2^-56 accumulate
- *                  exactly (FP32 integers in tensor memory, drained every 160 k into int64),
- *                  and each task's sum is rounded to FP64 once. Per element the error is
- *                  below 2^-48 * sum_k |a_ik| |b_kj| scaled by the row / column maxima
- *                  (about 1e-14 relative for random data); the tests and the benchmark
- *                  state the measured relative error against the FP64 result. Real and
+ *                  in tensor memory (FP32 integers, drained every 160 k into int64; exact but
+ *                  for the weights 2^-48 and 2^-56 where nearly all digits are at a limit),
+ *                  and each task's sum is rounded to FP64 once, ties to even. With s the
+ *                  power of two above row i's largest |a|, t that above column j's largest
+ *                  |b|, a task of k products (complex: 2 k) is off by at most
+ *                  (4.6 k + 172 ceil(k / 160)) 2^-49 s t before that rounding (at most 16
+ *                  of the 172 measured); for random data the whole result is within 2.5e-14
+ *                  relative of FP64's, as the tests and the benchmark state. Real and
  *                  complex128 tensors (a complex product runs as the real product of A's
  *                  interleaved parts with B's 2 x 2 real form); output blocks with n, k <= 8
  *                  stay on the FP64 pipe. */
@@ -113,7 +116,8 @@ typedef struct qltg_ctrct_plan qltg_ctrct_plan;
  * TensorContractionExecutor (reference tensor_manipulation/ten_ctrct.h:177-217): saved
  * axes, transpose orders, result legs = saved A legs ++ saved B legs, and the sector
  * pairing / task list of BlockSparseDataTensor::DataBlkGenForTenCtrct
- * (qltensor/blk_spar_data_ten/data_blk_operations.h:411-578), computed on the device.
+ * (qltensor/blk_spar_data_ten/data_blk_operations.h:411-578), computed on the host for
+ * small plans, else on the device.
  * Contracted legs must be inverse to each other (same sectors, opposite direction). */
 QLTG_API int qltg_ctrct_plan_create(qltg_ctx* ctx, const qltg_tensor_desc* a, const qltg_tensor_desc* b,
                            const int64_t* axes_a, const int64_t* axes_b, int32_t naxes,

@@ -246,8 +246,8 @@ void exec_contraction(CtrctPlan& p, const void* a, const void* b, void* c, int m
 // grouped GEMM launchers (gemm_f64.cu)
 constexpr int kF64TileCols = 16;   // columns of an FP64 warp tile
 bool skinny_cblk(const GemmSchedule& g, int32_t q);
-// Grid of the skinny kernel: one full wave of resident CTAs (the first call queries the
-// occupancy; call it once outside any stream capture).
+// Grid of the skinny kernel: one full wave of resident CTAs, up to four for complex (the first
+// call queries the occupancy; call it once outside any stream capture).
 int skinny_grid(int items, bool cplx, int num_sms);
 // Operand buffers of one execution: scratch (transposed blocks) and source (the operands as
 // passed in, for blocks flagged kFromSrc).

@@ -11,7 +11,7 @@
 //  * k_gemm_f64    - FP64 / complex128 (4 real FMAs per complex FMA) on warp tiles. On this
 //                    GPU the FP64 tensor path (mma.sync m8n8k4 f64) runs at the same rate as
 //                    DFMA (about 1.05 TFLOP/s each, measured) but pads every block to 8 x 8 x 4
-//                    fragments, so predicated DFMA is the faster FP64 kernel;
+//                    fragments, so DFMA, with nothing predicated, is the faster FP64 kernel;
 //  * k_gemm_skinny - output blocks with n <= 8 and k <= 8 (the MPO steps of the two-site
 //                    matvec: m up to 3e4, k, n <= 3): one output per lane, memory-streaming.
 #include <algorithm>

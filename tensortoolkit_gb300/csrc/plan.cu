@@ -1,4 +1,4 @@
-// Contraction planning: sector pairing on the device.
+// Contraction planning: sector pairing, on the host for small plans, else on the device.
 //
 // The reference builds the task list on the host with an O(nA * nB) double loop comparing
 // VecPartHasher values of the contracted block coordinates
